@@ -411,6 +411,7 @@ Gridder::~Gridder() {
   for (auto& e : piece_pass_)
     if (e) cudaEventDestroy(e);
   if (piece_binned_) cudaEventDestroy(piece_binned_);
+  if (legacy_ev_) cudaEventDestroy(legacy_ev_);
   if (stream_) {
     cudaStreamSynchronize(stream_);
     cudaStreamDestroy(stream_);
@@ -1203,6 +1204,14 @@ void Gridder::degrid_plan(Chunk& dc, Plan& pl) {
 // ---------------------------------------------------------------------------
 // finalise / initialise degrid
 // ---------------------------------------------------------------------------
+// Device buffers of the caller are read and written on the handle's own
+// stream, after the work that the caller has put on the legacy default stream.
+void Gridder::order_after_legacy_stream() {
+  if (!legacy_ev_) cuda_check(cudaEventCreateWithFlags(&legacy_ev_, cudaEventDisableTiming), "event");
+  cuda_check(cudaEventRecord(legacy_ev_, cudaStreamLegacy), "event");
+  cuda_check(cudaStreamWaitEvent(stream_, legacy_ev_, 0), "wait default stream");
+}
+
 void Gridder::prepare_corrections() {
   // SphFuncVisGridder::correctConvolution factors for the padded shape; the
   // AWProject gridder applies them only with a spheroidal taper
@@ -1212,31 +1221,24 @@ void Gridder::prepare_corrections() {
     return;
   }
   const int support = (kind_ == Kind::SphFunc) ? sph_support_ : 3;
-  Spheroidal g(M_PI * support, alpha_);
-  std::vector<double> cx = sph_correction(nx_, g), cy = sph_correction(ny_, g);
   cuda_check(corr_d_.ensure((nx_ + ny_) * sizeof(double)), "alloc");
-  cuda_check(cudaMemcpy(corr_d_.p, cx.data(), nx_ * sizeof(double), cudaMemcpyHostToDevice), "up");
-  cuda_check(cudaMemcpy(corr_d_.as<double>() + nx_, cy.data(), ny_ * sizeof(double), cudaMemcpyHostToDevice), "up");
-}
-
-static void extract_centre(const float* src, int snx, int sny, int nplanes, float* dst, int dnx, int dny, bool dst_dev,
-                           cudaStream_t st) {
-  const int x0 = (snx - dnx) / 2, y0 = (sny - dny) / 2;
-  for (int p = 0; p < nplanes; ++p) {
-    const float* s = src + (size_t)p * snx * sny + x0 + (size_t)snx * y0;
-    float* d = dst + (size_t)p * dnx * dny;
-    cuda_check(cudaMemcpy2DAsync(d, dnx * sizeof(float), s, snx * sizeof(float), dnx * sizeof(float), dny,
-                                 dst_dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st),
-               "extract");
-  }
+  rc_check(grid_correction(Spheroidal(M_PI * support, alpha_).series_tables(), nx_, ny_, corr_d_.as<double>(), stream_),
+           "grid correction");
 }
 
 void Gridder::finalise_grid(float* out, bool out_on_device) {
   throw_if(!grids_.p || nx_ == 0, YG_ERR_STATE, "finaliseGrid called before gridding");
+  order_after_legacy_stream();
   prepare_corrections();
   const int nplanes = npol_ * nchan_;
-  const long long total = (long long)nx_ * ny_ * nplanes;
-  cuda_check(img_tmp_.ensure(total * sizeof(float)), "alloc");
+  const int onx = (int)std::lround(nx_ / padding_), ony = (int)std::lround(ny_ / padding_);
+  throw_if(onx > nx_ || ony > ny_, YG_ERR_CUDA, "finaliseGrid: the padded grid is smaller than the image");
+  const size_t out_bytes = (size_t)onx * ony * nplanes * sizeof(float);
+  float* img = out;
+  if (!out_on_device) {
+    cuda_check(img_tmp_.ensure(out_bytes), "alloc");
+    img = img_tmp_.as<float>();
+  }
   std::vector<StackScreen> screens;
   const std::vector<StackScreen>* sp = nullptr;
   if (kind_ == Kind::WStack || kind_ == Kind::WStackWProject) {
@@ -1246,11 +1248,10 @@ void Gridder::finalise_grid(float* out, bool out_on_device) {
   }
   const double* cx = corr_d_.p ? corr_d_.as<double>() : nullptr;
   const double* cy = corr_d_.p ? corr_d_.as<double>() + nx_ : nullptr;
-  rc_check(image_finalise(fft_, grids_.as<float2>(), ngrids(), nx_, ny_, nplanes, sp, cx, cy, img_tmp_.as<float>(),
-                          stream_),
+  rc_check(image_finalise(fft_, grids_.as<float2>(), ngrids(), nx_, ny_, nplanes, sp, cx, cy, img, onx, ony, stream_),
            "finaliseGrid");
-  const int onx = (int)std::lround(nx_ / padding_), ony = (int)std::lround(ny_ / padding_);
-  extract_centre(img_tmp_.as<float>(), nx_, ny_, nplanes, out, onx, ony, out_on_device, stream_);
+  if (!out_on_device)
+    cuda_check(cudaMemcpyAsync(out, img, out_bytes, cudaMemcpyDeviceToHost, stream_), "download image");
   sync();
   if (clear_grids_) grids_.release();
 }
@@ -1308,16 +1309,23 @@ void Gridder::finalise_weights(float* out, bool out_on_device) {
       cuda_check(cudaMemcpy(out, dst, (size_t)onx * ony * np * sizeof(float), cudaMemcpyDeviceToHost), "weights");
     return;
   }
-  std::vector<float> h((size_t)onx * ony * npol_ * nchan_);
+  const size_t npix = (size_t)onx * ony;
+  std::vector<float> vals;
   for (int c = 0; c < nchan_; ++c)
     for (int p = 0; p < npol_; ++p) {
       double s = 0.0;
       for (int z = 0; z < rows; ++z) s += sw[z + (size_t)rows * (p + (size_t)npol_ * c)];
-      std::fill(h.begin() + (size_t)(p + npol_ * c) * onx * ony, h.begin() + (size_t)(p + npol_ * c + 1) * onx * ony,
-                (float)s);
+      vals.push_back((float)s);
     }
-  if (out_on_device) cuda_check(cudaMemcpy(out, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice), "weights");
-  else std::memcpy(out, h.data(), h.size() * sizeof(float));
+  if (out_on_device) {
+    // filled where it lies: building the image on the host and uploading it
+    // took 24 ms + the host fill for 4096^2 x 4
+    order_after_legacy_stream();
+    rc_check(fill_planes(out, (long long)npix, vals, stream_), "weights");
+    sync();
+  } else {
+    for (size_t p = 0; p < vals.size(); ++p) std::fill(out + p * npix, out + (p + 1) * npix, vals[p]);
+  }
 }
 
 void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int nchan, const float* image,
@@ -1329,37 +1337,21 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   const int nplanes = npol * nchan;
   const long long in_total = (long long)nx * ny * nplanes;
   const long long total = (long long)nx_ * ny_ * nplanes;
-  // model emptiness check on the host copy (or a device download)
-  std::vector<float> h;
-  const float* hp = image;
-  if (on_device) {
-    h.resize(in_total);
-    cuda_check(cudaMemcpy(h.data(), image, in_total * sizeof(float), cudaMemcpyDeviceToHost), "download model");
-    hp = h.data();
-  }
-  bool empty = true;
-  for (long long i = 0; i < in_total; ++i)
-    if (std::fabs(hp[i]) > 0.f) { empty = false; break; }
-  model_empty_ = empty;
   const size_t gbytes = (size_t)ngrids() * total * sizeof(float2);
   cuda_check(grids_.ensure(gbytes), "alloc grids");
-  if (empty) {
-    cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
-    sync();
-    return;
+  // the model image on the device: the caller's, or an upload of it; the
+  // first pass over it also tells whether it is empty
+  cuda_check(img_tmp_.ensure(64 + (on_device ? 0 : in_total * sizeof(float))), "alloc");
+  int* any = img_tmp_.as<int>();
+  const float* dimg = image;
+  if (on_device) {
+    order_after_legacy_stream();
+  } else {
+    float* up = img_tmp_.as<float>() + 16;
+    cuda_check(cudaMemcpyAsync(up, image, in_total * sizeof(float), cudaMemcpyHostToDevice, stream_), "upload model");
+    dimg = up;
   }
-  // padded model on the device
-  cuda_check(img_tmp_.ensure(total * sizeof(float) * 2), "alloc");
-  float* padded = img_tmp_.as<float>();
-  float* corrected = padded + total;
-  cuda_check(cudaMemsetAsync(padded, 0, total * sizeof(float), stream_), "memset");
-  const int x0 = (nx_ - nx) / 2, y0 = (ny_ - ny) / 2;
-  for (int p = 0; p < nplanes; ++p) {
-    cuda_check(cudaMemcpy2DAsync(padded + (size_t)p * nx_ * ny_ + x0 + (size_t)nx_ * y0, nx_ * sizeof(float),
-                                 image + (size_t)p * nx * ny, nx * sizeof(float), nx * sizeof(float), ny,
-                                 on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream_),
-               "upload model");
-  }
+  cuda_check(cudaMemsetAsync(any, 0, sizeof(int), stream_), "memset");
   prepare_corrections();
   std::vector<StackScreen> screens;
   const std::vector<StackScreen>* sp = nullptr;
@@ -1370,10 +1362,19 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   }
   const double* cx = corr_d_.p ? corr_d_.as<double>() : nullptr;
   const double* cy = corr_d_.p ? corr_d_.as<double>() + nx_ : nullptr;
-  rc_check(image_to_grids(fft_, padded, nx_, ny_, nplanes, sp, ngrids(), cx, cy, corrected, grids_.as<float2>(),
+  rc_check(image_to_grids(fft_, dimg, nx, ny, nx_, ny_, nplanes, sp, ngrids(), cx, cy, grids_.as<float2>(), any,
                           stream_),
            "initialiseDegrid");
+  int seen = 0;
+  cuda_check(cudaMemcpyAsync(&seen, any, sizeof(int), cudaMemcpyDeviceToHost, stream_), "model check");
   sync();
+  model_empty_ = seen == 0;
+  if (model_empty_) {
+    cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
+    sync();
+    return;
+  }
+  throw_if(nx > nx_ || ny > ny_, YG_ERR_CUDA, "initialiseDegrid: the padded grid is smaller than the image");
 }
 
 void Gridder::finalise_degrid() {

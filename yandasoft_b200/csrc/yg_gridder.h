@@ -191,6 +191,7 @@ class Gridder {
   void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
+  void order_after_legacy_stream();
   std::vector<uint8_t> psf_rows(const Chunk& hc);
 
   Kind kind_ = Kind::SphFunc;
@@ -288,6 +289,7 @@ class Gridder {
   void run_pieces(Chunk& c, bool degridding);
   ImageFFT fft_;
   cudaStream_t stream_ = nullptr;
+  cudaEvent_t legacy_ev_ = nullptr;
   Stats stats_;
   int device_ = 0;
   bool device_ready_ = false;

@@ -1,12 +1,14 @@
 // Image-side steps of the gridders on the GPU: finaliseGrid and
 // initialiseDegrid (askap/gridding/TableVisGridder.cc:1109-1236,1286-1319)
 // and the w-stack variants (askap/gridding/WStackVisGridder.cc:134-171,
-// 216-337).  Transforms are batched cuFFT C2C over all (pol, chan) planes with
-// the centred-transform checkerboard folded into the element-wise kernels;
-// the grid correction (SphFuncVisGridder::correctConvolution) is applied as
-// separable FP64 factors in the same pass.
+// 216-337).  Transforms are batched cuFFT C2C over all (pol, chan) planes; the
+// centring of both sides costs no pass of its own (k_image_accum,
+// k_image_to_uv), and the grid correction
+// (SphFuncVisGridder::correctConvolution) is applied as separable FP64 factors
+// in the same passes.
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -37,65 +39,189 @@ __device__ __forceinline__ bool wstack_screen(const StackScreen& s, int x, int y
   return true;
 }
 
-__global__ void k_sign_copy(const float2* __restrict__ in, float2* __restrict__ out, int nx, int ny, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-    const float s = sgn_in(x, y);
-    const float2 v = in[i];
-    out[i] = make_float2(v.x * s, v.y * s);
-  }
-}
-
-// acc (+)= real(out_sign * v [* screen])
-__global__ void k_accum_real(const float2* __restrict__ f, float* __restrict__ acc, int nx, int ny, long long total,
-                             int first, int use_screen, StackScreen scr) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-    const float s = sgn_out(x, y, nx, ny);
-    float2 v = f[i];
+// Backward side of a centred transform, fused with everything after it: with
+// B the plain backward FFT of a grid, the centred transform is
+//   (-1)^(x + nx/2 + y + ny/2) B[(x + nx/2) mod nx, (y + ny/2) mod ny],
+// so the grid goes into the FFT as it is (out of place; no checkerboard copy
+// of it) and the roll is this kernel's read index.  One thread per output
+// pixel walks the planes: the w-stack screen (FP64 square root, sine, cosine)
+// is evaluated once for all of them, and only the centre that is kept is read.
+//   acc (+)= real(B' [* screen]), and for the last grid times cx[x] cy[y].
+// HBM bound: 8 B read and 4 B (later grids 8 B) of image per pixel.  A grid of
+// 4096^2 x 4 planes: 698 us for checkerboard copy + accumulation before
+// (20 B more traffic, the screen per plane, 64-bit divisions per pixel).
+__global__ void __launch_bounds__(256) k_image_accum(const float2* __restrict__ f, float* __restrict__ acc, int nx,
+                                                     int ny, int onx, int ony, int nplanes, int first, int last,
+                                                     int use_screen, StackScreen scr, const double* __restrict__ cx,
+                                                     const double* __restrict__ cy) {
+  const int ox = blockIdx.x * blockDim.x + threadIdx.x;
+  const int oy = blockIdx.y;
+  if (ox >= onx) return;
+  const int x = ox + (nx - onx) / 2, y = oy + (ny - ony) / 2;
+  const int bx = x + nx / 2 < nx ? x + nx / 2 : x + nx / 2 - nx;
+  const int by = y + ny / 2 < ny ? y + ny / 2 : y + ny / 2 - ny;
+  const float s = sgn_out(x, y, nx, ny);
+  float cr = 1.f, ci = 0.f;
+  const bool inside = use_screen && wstack_screen(scr, x, y, &cr, &ci);
+  const double corr = (last && cx) ? cx[x] * cy[y] : 1.0;
+  const size_t in = bx + (size_t)nx * by, in_plane = (size_t)nx * ny;
+  const size_t o = ox + (size_t)onx * oy, o_plane = (size_t)onx * ony;
+#pragma unroll 4
+  for (int p = 0; p < nplanes; ++p) {
+    float2 v = f[in + p * in_plane];
     v.x *= s;
     v.y *= s;
     float r = v.x;
-    if (use_screen) {
-      float cr, ci;
-      if ((v.x != 0.f || v.y != 0.f) && wstack_screen(scr, x, y, &cr, &ci)) r = __fsub_rn(__fmul_rn(v.x, cr), __fmul_rn(v.y, ci));
+    if (inside && (v.x != 0.f || v.y != 0.f)) r = __fsub_rn(__fmul_rn(v.x, cr), __fmul_rn(v.y, ci));
+    float a = first ? r : __fadd_rn(acc[o + p * o_plane], r);
+    if (last && cx) a = (float)((double)a * corr);
+    acc[o + p * o_plane] = a;
+  }
+}
+
+// Forward side: the plain FFT of
+//   (-1)^(x' + y') a[(x' + nx/2) mod nx, (y' + ny/2) mod ny]
+// is the centred transform of a itself, both checkerboards included, so the
+// grids need no sign pass after the FFT.  a is the image in the centre of the
+// padded plane, corrected, and with w-stacks conj(image * screen) (the screen
+// once per pixel for all planes).  HBM bound: 4 B read, 8 B written per cell;
+// 507 us per grid of 4096^2 x 4 planes before with the sign pass (16 B more).
+__global__ void __launch_bounds__(256) k_image_to_uv(const float* __restrict__ img, float2* __restrict__ out, int inx,
+                                                     int iny, int nx, int ny, int nplanes, int use_screen,
+                                                     StackScreen scr, const double* __restrict__ cx,
+                                                     const double* __restrict__ cy, int* __restrict__ any) {
+  const int bx = blockIdx.x * blockDim.x + threadIdx.x;
+  const int by = blockIdx.y;
+  bool seen = false;
+  if (bx < nx) {
+    const int x = bx + nx / 2 < nx ? bx + nx / 2 : bx + nx / 2 - nx;
+    const int y = by + ny / 2 < ny ? by + ny / 2 : by + ny / 2 - ny;
+    const int ix = x - (nx - inx) / 2, iy = y - (ny - iny) / 2;
+    const bool on = ix >= 0 && iy >= 0 && ix < inx && iy < iny;
+    float cr = 1.f, ci = 0.f;
+    const bool inside = use_screen && wstack_screen(scr, x, y, &cr, &ci);
+    const double corr = cx ? cx[x] * cy[y] : 1.0;
+    const float s = sgn_in(bx, by);
+    const size_t in = on ? ix + (size_t)inx * iy : 0, in_plane = (size_t)inx * iny;
+    const size_t o = bx + (size_t)nx * by, o_plane = (size_t)nx * ny;
+#pragma unroll 4
+    for (int p = 0; p < nplanes; ++p) {
+      float v = on ? img[in + p * in_plane] : 0.f;
+      seen = seen || fabsf(v) > 0.f;
+      if (cx) v = (float)((double)v * corr);
+      float2 c = make_float2(v, 0.f);
+      if (use_screen) {
+        if (inside && v != 0.f) c = make_float2(__fmul_rn(v, cr), __fmul_rn(v, ci));
+        c.y = -c.y;
+      }
+      out[o + p * o_plane] = make_float2(c.x * s, c.y * s);
     }
-    acc[i] = first ? r : __fadd_rn(acc[i], r);
   }
+  if (any && __syncthreads_or(seen) && threadIdx.x == 0) *any = 1;
 }
 
-// img *= ccfx[x] * ccfy[y] (FP64 factors, FP32 result)
-__global__ void k_correct(float* __restrict__ img, const double* __restrict__ cx, const double* __restrict__ cy,
-                          int nx, int ny, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-    img[i] = (float)((double)img[i] * (cx[x] * cy[y]));
+// Spheroidal function of one nu (Spheroidal::operator(), the same recurrence).
+__device__ double sph_value(const SphSeries& t, double nu) {
+  if (!(fabs(nu) < 1.0)) return 0.0;
+  const double s = sqrt(fmax(0.0, 1.0 - nu * nu));
+  double pmm = sqrt(0.5);
+  for (int k = 0; k < t.m; ++k) pmm = -pmm * t.pmm[k] * s;
+  double sum = t.coeff[0] * pmm;
+  double prev = pmm, cur = nu * sqrt(2.0 * t.m + 3.0) * pmm;
+  for (int q = 0; q < 2 * (t.nterms - 1) - 1; ++q) {
+    const double next = t.a[q] * (nu * cur - t.b[q] * prev);
+    prev = cur;
+    cur = next;
+    if ((q & 1) == 0) sum += t.coeff[q / 2 + 1] * next;
   }
+  return sum / t.sum0 * pow(1.0 - nu * nu, -t.alpha / 2.0);
 }
 
-// image (already corrected) -> in_sign * [conj](complex(img) [* screen])
-__global__ void k_image_to_c(const float* __restrict__ img, float2* __restrict__ out, int nx, int ny, long long total,
-                             int use_screen, StackScreen scr) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-    float2 v = make_float2(img[i], 0.f);
-    if (use_screen) {
-      float cr, ci;
-      if (v.x != 0.f && wstack_screen(scr, x, y, &cr, &ci)) v = make_float2(__fmul_rn(v.x, cr), __fmul_rn(v.x, ci));
-      v.y = -v.y;
+// Correction factors of one axis per block: the spheroidal over the axis
+// (single precision, edge interpolated), low-passed to its central 2 * 3 + 1
+// Fourier coefficients, scaled to keep the centre, inverted.  Only those seven
+// coefficients exist after the filter, so they are summed directly (n terms
+// each) and the filtered function is their seven-term series: 14 n instead of
+// two transforms, for any n.  Latency bound: two blocks.  Before, on the host
+// with two uploads: 0.3 ms at 1024^2, and a plain n^2 transform at sizes that
+// are not a power of two (590 ms at 3000^2).
+__global__ void __launch_bounds__(1024) k_grid_correction(const __grid_constant__ SphSeries t, int nx, int ny,
+                                                          double* __restrict__ corr) {
+  __shared__ double part[32][7];
+  __shared__ double coef[7];
+  const int n = blockIdx.x == 0 ? nx : ny;
+  double* d = corr + (blockIdx.x == 0 ? 0 : nx);
+  const int half = n / 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n; i += blockDim.x) d[i] = (double)(float)sph_value(t, fabs((double)(i - half)) / (double)half);
+  __syncthreads();
+  if (tid == 0 && n > 3) {
+    const float e = __fadd_rn(__fmul_rn(3.0f, __fsub_rn((float)d[1], (float)d[2])), (float)d[3]);
+    d[0] = (double)e;
+    if (n % 2 == 1) d[n - 1] = (double)e;
+  }
+  __syncthreads();
+  // sums of v cos(2 pi k j / n), k = 0..3, and v sin, k = 1..3, j = i - half
+  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+  for (int i = tid; i < n; i += blockDim.x) {
+    const double v = d[i], x = 2.0 * (double)(i - half) / (double)n;
+    acc[0] += v;
+#pragma unroll
+    for (int k = 1; k <= 3; ++k) {
+      double sn, cs;
+      sincospi(k * x, &sn, &cs);
+      acc[k] += v * cs;
+      acc[3 + k] += v * sn;
     }
-    const float s = sgn_in(x, y);
-    out[i] = make_float2(v.x * s, v.y * s);
+  }
+#pragma unroll
+  for (int q = 0; q < 7; ++q) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
+    if (lane == 0) part[warp][q] = acc[q];
+  }
+  __syncthreads();
+  if (tid < 7) {
+    double sum = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += part[w][tid];
+    coef[tid] = sum;
+  }
+  const double centre = d[half];
+  __syncthreads();
+  // coefficient k is (coef[|k|], -sign(k) coef[3 + |k|]); indices half + k
+  const int klo = max(-3, -half), khi = min(3, n - 1 - half);
+  double c0r = 0.0, c0i = 0.0;
+  for (int k = klo; k <= khi; ++k) {
+    c0r += coef[abs(k)];
+    if (k != 0) c0i += k > 0 ? -coef[3 + k] : coef[3 - k];
+  }
+  const double c2 = c0r * c0r + c0i * c0i;
+  const double nr = centre * c0r / c2, ni = -centre * c0i / c2;      // centre / filtered centre
+  for (int i = tid; i < n; i += blockDim.x) {
+    const double x = 2.0 * (double)(i - half) / (double)n;
+    double vr = 0.0, vi = 0.0;
+    for (int k = klo; k <= khi; ++k) {
+      double sn, cs;
+      sincospi(k * x, &sn, &cs);
+      const double fr = coef[abs(k)], fi = k == 0 ? 0.0 : (k > 0 ? -coef[3 + k] : coef[3 - k]);
+      vr += fr * cs - fi * sn;
+      vi += fr * sn + fi * cs;
+    }
+    const double v = vr * nr - vi * ni;
+    d[i] = fabs(v) > 1e-10 ? 1.0 / v : 0.0;
   }
 }
 
-__global__ void k_sign_out(float2* __restrict__ g, int nx, int ny, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-    const float s = sgn_out(x, y, nx, ny);
-    const float2 v = g[i];
-    g[i] = make_float2(v.x * s, v.y * s);
-  }
+// vals by value: up to 32 planes per launch
+struct PlaneValues {
+  float v[32];
+};
+
+__global__ void k_fill_planes(float* __restrict__ out, long long npix, const __grid_constant__ PlaneValues vals) {
+  const float v = vals.v[blockIdx.y];
+  float* o = out + (size_t)blockIdx.y * npix;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npix; i += (long long)gridDim.x * blockDim.x)
+    o[i] = v;
 }
 
 static int blocks_for(long long total) {
@@ -136,44 +262,58 @@ ImageFFT::~ImageFFT() {
   if (plan_ok) cufftDestroy(plan);
 }
 
-// image[nx, ny, nplanes] = sum_g real(backward FFT(grid_g) [* screen_g]) * corr
-int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny, int nplanes,
-                   const std::vector<StackScreen>* screens, const double* corr_x, const double* corr_y, float* out,
-                   cudaStream_t st) {
-  int rc = f.ensure(nx, ny, nplanes, st);
-  if (rc) return rc;
-  const long long total = (long long)nx * ny * nplanes;
-  for (int g = 0; g < ngrids; ++g) {
-    k_sign_copy<<<blocks_for(total), 256, 0, st>>>(grids + (size_t)g * total, f.work.as<float2>(), nx, ny, total);
-    if (cufftExecC2C(f.plan, (cufftComplex*)f.work.p, (cufftComplex*)f.work.p, CUFFT_INVERSE) != CUFFT_SUCCESS)
-      return YG_ERR_CUDA;
-    StackScreen s{};
-    const bool use = screens != nullptr;
-    if (use) s = (*screens)[g];
-    k_accum_real<<<blocks_for(total), 256, 0, st>>>(f.work.as<float2>(), out, nx, ny, total, g == 0, use, s);
-  }
-  if (corr_x && corr_y) k_correct<<<blocks_for(total), 256, 0, st>>>(out, corr_x, corr_y, nx, ny, total);
+int grid_correction(const SphSeries& t, int nx, int ny, double* corr, cudaStream_t st) {
+  k_grid_correction<<<2, 1024, 0, st>>>(t, nx, ny, corr);
   IM_TRY(cudaGetLastError());
   return YG_OK;
 }
 
-// grids_g = forward FFT(in_sign * [conj](corr * image [* screen_g]))
-int image_to_grids(ImageFFT& f, const float* image, int nx, int ny, int nplanes,
-                   const std::vector<StackScreen>* screens, int ngrids, const double* corr_x, const double* corr_y,
-                   float* corrected_tmp, float2* grids, cudaStream_t st) {
+int fill_planes(float* out, long long npix, const std::vector<float>& vals, cudaStream_t st) {
+  for (size_t p0 = 0; p0 < vals.size(); p0 += 32) {
+    PlaneValues v{};
+    const int n = (int)std::min<size_t>(32, vals.size() - p0);
+    for (int i = 0; i < n; ++i) v.v[i] = vals[p0 + i];
+    const int blocks = (int)std::max(1ll, std::min((npix + 255) / 256, 148ll * 8));
+    k_fill_planes<<<dim3(blocks, n), 256, 0, st>>>(out + p0 * npix, npix, v);
+  }
+  IM_TRY(cudaGetLastError());
+  return YG_OK;
+}
+
+int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny, int nplanes,
+                   const std::vector<StackScreen>* screens, const double* corr_x, const double* corr_y, float* out,
+                   int onx, int ony, cudaStream_t st) {
   int rc = f.ensure(nx, ny, nplanes, st);
   if (rc) return rc;
   const long long total = (long long)nx * ny * nplanes;
-  IM_TRY(cudaMemcpyAsync(corrected_tmp, image, total * sizeof(float), cudaMemcpyDeviceToDevice, st));
-  if (corr_x && corr_y) k_correct<<<blocks_for(total), 256, 0, st>>>(corrected_tmp, corr_x, corr_y, nx, ny, total);
+  const bool corr = corr_x && corr_y;
+  for (int g = 0; g < ngrids; ++g) {
+    if (cufftExecC2C(f.plan, (cufftComplex*)(grids + (size_t)g * total), (cufftComplex*)f.work.p, CUFFT_INVERSE) !=
+        CUFFT_SUCCESS)
+      return YG_ERR_CUDA;
+    const bool use = screens != nullptr;
+    k_image_accum<<<dim3((onx + 255) / 256, ony), 256, 0, st>>>(
+        f.work.as<float2>(), out, nx, ny, onx, ony, nplanes, g == 0, g == ngrids - 1, use,
+        use ? (*screens)[g] : StackScreen{}, corr ? corr_x : nullptr, corr_y);
+  }
+  IM_TRY(cudaGetLastError());
+  return YG_OK;
+}
+
+int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, int ny, int nplanes,
+                   const std::vector<StackScreen>* screens, int ngrids, const double* corr_x, const double* corr_y,
+                   float2* grids, int* any, cudaStream_t st) {
+  int rc = f.ensure(nx, ny, nplanes, st);
+  if (rc) return rc;
+  const long long total = (long long)nx * ny * nplanes;
+  const bool corr = corr_x && corr_y;
   for (int g = 0; g < ngrids; ++g) {
     float2* dst = grids + (size_t)g * total;
-    StackScreen s{};
     const bool use = screens != nullptr;
-    if (use) s = (*screens)[g];
-    k_image_to_c<<<blocks_for(total), 256, 0, st>>>(corrected_tmp, dst, nx, ny, total, use, s);
+    k_image_to_uv<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(image, dst, inx, iny, nx, ny, nplanes, use,
+                                                             use ? (*screens)[g] : StackScreen{},
+                                                             corr ? corr_x : nullptr, corr_y, g == 0 ? any : nullptr);
     if (cufftExecC2C(f.plan, (cufftComplex*)dst, (cufftComplex*)dst, CUFFT_FORWARD) != CUFFT_SUCCESS) return YG_ERR_CUDA;
-    k_sign_out<<<blocks_for(total), 256, 0, st>>>(dst, nx, ny, total);
   }
   IM_TRY(cudaGetLastError());
   return YG_OK;

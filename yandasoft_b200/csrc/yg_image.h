@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "yg_internal.h"
+#include "yg_spheroidal.h"
 
 namespace yg {
 
@@ -25,12 +26,24 @@ struct ImageFFT {
   ~ImageFFT();
 };
 
+// Correction factors of SphFuncVisGridder::correctConvolution
+// (SphFuncVisGridder.cc:171-248): corr[0, nx) along x, corr[nx, nx + ny) along y.
+int grid_correction(const SphSeries& t, int nx, int ny, double* corr, cudaStream_t st);
+
+// out (onx, ony, nplanes), device: the centre of
+// corr_x corr_y sum_g real(backward FFT(grid_g) [* screen_g]) over (nx, ny)
 int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny, int nplanes,
                    const std::vector<StackScreen>* screens, const double* corr_x, const double* corr_y, float* out,
-                   cudaStream_t st);
-int image_to_grids(ImageFFT& f, const float* image, int nx, int ny, int nplanes,
+                   int onx, int ony, cudaStream_t st);
+// grids_g = forward FFT of the device image (inx, iny, nplanes) in the centre
+// of (nx, ny), corrected, times screen_g; *any (device) is set when a pixel is
+// not zero
+int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, int ny, int nplanes,
                    const std::vector<StackScreen>* screens, int ngrids, const double* corr_x, const double* corr_y,
-                   float* corrected_tmp, float2* grids, cudaStream_t st);
+                   float2* grids, int* any, cudaStream_t st);
+
+// every pixel of plane p of out (npix per plane, device) = vals[p]
+int fill_planes(float* out, long long npix, const std::vector<float>& vals, cudaStream_t st);
 
 // AWProject finaliseWeights: planes[r] = CF index of sum-of-weights row r with
 // data, offs[r] its CF offset, wts[r * nplanes + pol + npol * chan] its
