@@ -165,16 +165,18 @@ void yg_plan_destroy(yg_plan* plan);
 /* ---- tuning ---- */
 int yg_set_tile(yg_gridder* g, int32_t tile);      /* 0 = automatic */
 int yg_set_item_size(yg_gridder* g, int32_t vmax); /* samples per work item */
-/* k_grid thread layout: 0 or 1 the default, 2 and 3 halve / quarter the tap
+/* Record order and thread layout of the grid kernels: 0 the default
+ * (plane-major for AWProject, CF-major for the others), 1 CF-major, 2 and 3
+ * halve / quarter the tap
  * threads (each steps down twice / four times the rows); YG_ERR_UNSUPPORTED
  * at the next grid call when the CF width has no such layout.  Adding 16
  * keeps each thread's running tap sums in registers while consecutive
  * samples cover the same cell (layouts of at most 8 rows per thread); adding
  * 32 as well orders each tile's samples by position before CF for gridding
  * (plans made afterwards keep both orders) and reads the taps through L2;
- * adding 64 orders them by CF plane, then position, then oversampling offset
- * and stages each plane's offsets in shared memory once (16-wide CFs), and
- * 128 with it keeps that kernel's tile in global memory (two CTAs per SM).
+ * 64 (the other bits up to 128 are then ignored) orders them by CF plane, then
+ * position, then oversampling offset and keeps each footprint's running sums in
+ * registers (k_grid_pl; CFs of one common size).
  * Adding 256 degrids 16-wide CFs with the CF read per tap from the segment
  * ring (k_degrid_t) instead of the default register-held CF column; adding
  * 512 has the default degrid one sample per half-warp pass instead of two. */

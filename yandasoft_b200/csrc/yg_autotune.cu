@@ -71,14 +71,12 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   std::vector<int> vmaxes = {def_vmax};
   for (int v : {def_vmax / 4, def_vmax * 4})
     if (v >= 128 && v <= (1 << 20)) vmaxes.push_back(v);
-  // thread layouts: the default; for 16-wide CFs the plane-major records with
-  // staged CF planes (tile in global memory, 193, or in shared memory, 65;
-  // two polarisation groups, 194), half the threads, tap sums in registers
-  // over the CF-major records (17); for wider CFs the default, 17 and half
-  // the threads.  Position-major records with taps through L2 (32) measured
-  // slower on the benchmark workloads and are not tried.
-  const std::vector<int> variants =
-      wpad == 16 ? std::vector<int>{1, 193, 65, 194, 2, 17} : std::vector<int>{1, 17, 2};
+  // record orders and thread layouts: the CF-major kernel (1), the plane-major
+  // kernel (64), half the CF-major kernel's threads (2) and its tap sums in
+  // registers (17).  Position-major records with taps
+  // through L2 (32) measured slower on the benchmark workloads and are not
+  // tried.
+  const std::vector<int> variants{1, 64, 17, 2};
   const int save_tile = tile_override_, save_vmax = vmax_, save_mode = grid_mode_;
   Chunk scratch_chunk = dc;
   DevBuf model;

@@ -1,0 +1,17 @@
+// Plane-major gridding (k_grid_pl).
+#pragma once
+#include "yg_internal.h"
+
+namespace yg {
+
+// How the plane-major kernel takes this CF table: 0, not at all (matrices of
+// several sizes); n > 0, blocks of n consecutive matrices staged
+// in shared memory; -n, planes of n matrices read through L1 / L2.  |n| is the
+// number of matrices that the plane-major order treats as one CF plane.
+int grid_pl_block(const CFView& cf, int os, int cf_mode, int npol);
+
+// Grids the plane-major records of a plan (pl.rec_pos, pl.pl_fs).
+int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
+                 DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1);
+
+}  // namespace yg

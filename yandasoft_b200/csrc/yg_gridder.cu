@@ -16,6 +16,7 @@
 //                                           TableVisGridder.cc:997-1079,1109-1319,1381-1405
 //   FrequencyMapper::setupImage / setupMapping  FrequencyMapper.cc:55-107
 #include "yg_gridder.h"
+#include "yg_grid_pl.h"
 
 #include <algorithm>
 #include <cctype>
@@ -815,11 +816,19 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   // 16-wide CFs grid with residue rows modulo their real width (exact rows)
   // unless a layout of several slots per thread was asked for
   const int wpad16 = ((2 * smax + 1) + 15) / 16 * 16;
-  // (the plane-major kernel keeps exact rows with every layout)
-  a.wy = (wpad16 == 16 && ((grid_variant() & 15) <= 1 || (grid_variant() & 64)) && exact_rows_) ? 2 * smax + 1 : 0;
-  a.pos_major = (grid_variant() & 64) ? 2 : ((grid_variant() & 32) ? 1 : 0);
+  const int variant = grid_variant();
+  a.wy = (wpad16 == 16 && ((variant & 15) <= 1 || (variant & 64)) && exact_rows_) ? 2 * smax + 1 : 0;
+  // Records for the plane-major kernel where it takes the table: asked for by
+  // bit 64, or the automatic choice for AWProject.  The other gridders' images
+  // are divided by the spheroidal, whose factors of 10^4 in the corners turn
+  // the rounding of another order of a cell's sum into 1e-4 of the image: their
+  // automatic choice keeps the CF-major order, so that an image stays what it
+  // was bit for bit, and the plane-major order is theirs to ask for or tune to.
+  const bool planes = (variant & 64) || ((variant & 255) == 0 && kind_ == Kind::AWProject && !aw_taper_);
+  a.pl_fs = planes && cf_form_ == 0 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
+  a.pos_major = a.pl_fs != 0 ? 2 : ((variant & 32) && !(variant & 64) ? 1 : 0);
   a.key_planes = 0;
-  a.need_inv = 1;
+  a.need_inv = a.keep_inv = 1;
   a.ntx = (nx_ + a.tile - 1) / a.tile;
   a.nty = (ny_ + a.tile - 1) / a.tile;
   int mb = 0;
@@ -887,12 +896,9 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   fill_bin_args(a, dc, pl.chanmap.as<int>(), row_ok);
   if (use == PLAN_DEGRID) a.pos_major = 0;
   // a gridding-only plan for the plane-major kernel sorts once, by its key
-  const int wpad_b = ((cf_.maxsize + 15) / 16) * 16;
-  a.key_planes = (use == PLAN_GRID && a.pos_major == 2 && wpad_b == 16 && a.wy > 0 && a.wy <= 16 &&
-                  !cf_.view().varsup && dc.npol <= 4 && cf_form_ == 0)
-                     ? 1
-                     : 0;
-  a.need_inv = (use != PLAN_DEGRID && !a.key_planes) ? 1 : 0;
+  a.key_planes = (use == PLAN_GRID && a.pos_major == 2) ? 1 : 0;
+  a.keep_inv = use != PLAN_DEGRID ? 1 : 0;
+  a.need_inv = (use != PLAN_DEGRID && a.pos_major != 2) ? 1 : 0;
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;

@@ -18,10 +18,8 @@
 //                  the cells of a fixed residue class (x mod W, y mod W), so no
 //                  two threads ever touch the same cell (no atomics); its
 //                  weighted visibilities come from k_gather_cube.
-//   k_grid_pl      the same over plane-major records, each CF plane's
-//                  oversampling offsets staged in shared memory once, running
-//                  sums in registers, the tile in shared or global memory; its
-//                  producer warp forms the weighted visibilities itself.
+//   k_grid_pl      (yg_grid_pl.cu) over plane-major records, running sums in
+//                  registers.
 //   k_halo_sum     each output tile adds, in a fixed order, the overlapping
 //                  parts of its neighbours' padded tiles: deterministic, and
 //                  the grid is written once.
@@ -36,8 +34,11 @@
 #include <atomic>
 #include <cstdio>
 
+#include "yg_cf.h"
+#include "yg_grid_pl.h"
 #include "yg_internal.h"
 #include "yg_mlp.cuh"
+#include "yg_ring.cuh"
 #include "yg_sort.h"
 
 namespace yg {
@@ -145,7 +146,7 @@ __global__ void k_bin(BinArgs a, unsigned long long* __restrict__ key, unsigned 
                 const unsigned int m = morton2((unsigned)(iuo - tx * a.tile), (unsigned)(ivo - ty * a.tile));
                 if (a.key_planes) {
                   // plane-major: tile, CF plane, position, oversampling offset
-                  const unsigned long long os2 = (unsigned long long)a.os * a.os;
+                  const unsigned long long os2 = (unsigned)abs(a.pl_fs);
                   const unsigned long long cp = (unsigned)cfi / os2, fr = (unsigned)cfi % os2;
                   k = (((((unsigned long long)(gc * ntiles + tile) * ((unsigned long long)a.cf.ncf / os2) + cp)
                          << a.mbits) | m) * os2) + fr;
@@ -214,52 +215,13 @@ __global__ void k_fill_items(const int* __restrict__ tstart, const int* __restri
 }
 
 // ---------------------------------------------------------------------------
-// weights: rVis = phasor * conj(vis) * wt (* mfs), TableVisGridder.cc:775-806
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float noise_weight(float nre) {
-  const float vn = __fmul_rn(nre, nre);
-  return (vn > 0.f) ? (float)(1.0 / (double)vn) : 0.f;
-}
-
-__device__ __forceinline__ void phasor_of(const VisArgs& v, long long row, int chan, float* pr, float* pi) {
-  if (!v.delay) {
-    *pr = 1.f;
-    *pi = 0.f;
-    return;
-  }
-  const double ph = __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(2.0, kPi), v.freq[chan]), v.delay[row]), kC);
-  *pr = (float)cos(ph);
-  *pi = (float)sin(ph);
-}
-
-// rVis = phasor * conj(vis) * wt (* mfs) of sample s, polarisation p
-// (TableVisGridder.cc:775-806), wt (* mfs) for the PSF, wt for the
-// preconditioner function; FP32 with explicit rounding.
-__device__ __forceinline__ float2 weighted_vis(const VisArgs& v, long long s, long long n, int p, float pr, float pi,
-                                               float m) {
-  const float nre = v.noise ? v.noise[s + n * p].x : 1.f;
-  const float wt = noise_weight(nre);
-  if (v.pcf) return make_float2(__fmul_rn(1.f, wt), __fmul_rn(0.f, wt));
-  if (v.psf) return make_float2(__fmul_rn(__fmul_rn(1.f, wt), m), __fmul_rn(__fmul_rn(0.f, wt), m));
-  const float2 vv = v.vis[s + n * p];
-  const float vr = vv.x, vi = -vv.y;
-  float rr = __fsub_rn(__fmul_rn(pr, vr), __fmul_rn(pi, vi));
-  float ri = __fadd_rn(__fmul_rn(pr, vi), __fmul_rn(pi, vr));
-  rr = __fmul_rn(__fmul_rn(rr, wt), m);
-  ri = __fmul_rn(__fmul_rn(ri, wt), m);
-  return make_float2(rr, ri);
-}
-
-
-// ---------------------------------------------------------------------------
 // k_grid
 // ---------------------------------------------------------------------------
 struct GridKArgs {
   const int4* items;
   const unsigned int* val;   // sample ids, sorted
   const int4* rec;           // per sorted sample: cell, residues|w, cf index, sample id
-  const float2* svis;        // per sorted sample: npol weighted visibilities (k_grid_pl: null,
-                             // its producer forms them from the cube itself)
+  const float2* svis;        // per sorted sample: npol weighted visibilities
   const unsigned int* pos;   // iu | iv << 16, unsorted (by sample id)
   const int* cfi;            // unsorted
   VisArgs v;
@@ -287,78 +249,11 @@ struct GridKArgs {
 
 constexpr int kGridThreads = 256;
 constexpr int kBatch = 64;
-// bounded mbarrier waits: a wait gives up after 4 s on the global timer (and
-// after 2^26 polls, should the timer not advance)
-constexpr unsigned long long kWaitNs = 4000000000ull;
-constexpr long long kWaitPolls = 1ll << 26;
-
 struct VisRec {
   int cb;            // footprint origin cell (px0 + P py0) in the padded tile
   int mx, my;        // px0 mod W, py0 mod W
   int w;             // 2S+1 of this CF
 };
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-// one-dimensional TMA bulk copy global -> shared, completion on the mbarrier
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned phase) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// try_wait that may suspend the thread up to hint_ns while the phase is open
-__device__ __forceinline__ bool mbar_try_wait_for(unsigned long long* bar, unsigned phase, unsigned hint_ns) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// bounded wait; false when the limit was reached.  The bound is time, not a
-// poll count: CTAs of many kernels sharing the SMs (the major-cycle graph runs
-// instances side by side) can make an ordinary wait last many polls.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned phase) {
-  if (mbar_try_wait(bar, phase)) return true;
-  const unsigned long long t0 = global_ns();
-  for (long long i = 0; i < kWaitPolls; ++i) {
-    if (mbar_try_wait_for(bar, phase, 100000u)) return true;
-    if (global_ns() - t0 > kWaitNs) return false;
-  }
-  return false;
-}
 
 __host__ __device__ __forceinline__ unsigned cf_bytes(int w) { return (unsigned)(((w * w * 8) + 15) & ~15); }
 
@@ -368,8 +263,6 @@ __host__ __device__ __forceinline__ unsigned cf_bytes(int w) { return (unsigned)
 // Wp x Wp, brought in by a TMA bulk copy), the samples' records and
 // visibilities, and a header {count, index of the segment's first sample in
 // the item}.  count < 0 marks the end of the item.
-constexpr int kSeg = 32;
-
 __host__ __device__ __forceinline__ int seg_stage_bytes(int cfbuf, int npol) {
   return (cfbuf + kSeg * 16 + kSeg * npol * 8 + 16 + 127) / 128 * 128;
 }
@@ -382,10 +275,6 @@ static int min_stages_two_ctas(size_t stage) { return stage >= 8192 ? 2 : 4; }
 // dynamic shared memory per CTA with three CTAs per SM (228 kB per SM, 1 kB
 // reserved per CTA, a little kept for the static variables)
 constexpr size_t kSmem3Ctas = 75 * 1024 - 128;
-
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // Producer warp: walks the item's sorted samples 32 at a time (records and
 // visibilities loaded one window ahead), cuts each window at CF changes and
@@ -879,289 +768,6 @@ __global__ void __launch_bounds__(CFM >= 2 ? 288 : 544) k_grid(GridKArgs a) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// k_grid_pl: gridding of one work item whose samples are in plane-major order
-// (CF plane, then position in the tile, then oversampling offset), for
-// 16-wide CFs with exact residue rows (thread t owns x residue t mod 16 and
-// the y residues t / 16 + RY q < Wy of its SL slots, RY = ceil(Wy / SL)).  The producer warp stages records and
-// visibilities in segments of up to 32 samples of one CF plane and, when a
-// segment starts a new plane, brings every oversampling offset of that plane
-// (rows 0..Wy-1 of each padded CF, os^2 bulk copies) into one plane buffer,
-// after all earlier segments are consumed.  Consecutive samples of a plane
-// mostly cover the same cells, so each thread keeps its cell's running sums
-// in registers and adds them into the shared-memory tile only when a sample
-// moves it to another cell of its residue class (GridKernel::grid's sums,
-// GridKernel.cc:57-97, in another order).
-// ---------------------------------------------------------------------------
-template <int NPOL, int SL, int NG, bool GT>
-__global__ void __launch_bounds__(544) k_grid_pl(GridKArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int nthr = blockDim.x - 32;
-  const int ncw = nthr / 32;
-  const int Pg = a.Pg, Wy = a.Wy, os2 = a.pps;       // pps carries os^2 in this kernel
-  const int PG2 = Pg * Pg + nthr;
-  // GT: the padded tile lives in this item's scratch slot in global memory
-  // (L2), written only by the rare flushes, as reductions; shared memory then
-  // holds the plane buffer and the ring only (two CTAs per SM)
-  float2* acc_s = GT ? a.scratch + ((size_t)blockIdx.x * a.npol_total + a.pol0) * PG2
-                     : reinterpret_cast<float2*>(smem_raw);
-  size_t off = GT ? 0 : ((size_t)NPOL * PG2 * sizeof(float2) + 127) & ~(size_t)127;
-  float2* planebuf = reinterpret_cast<float2*>(smem_raw + off);
-  const int prow = Wy * 16;                           // float2 per oversampling offset
-  off += ((size_t)os2 * prow * sizeof(float2) + 127) & ~(size_t)127;
-  unsigned char* ring = smem_raw + off;
-  const int SB = a.stage_bytes, NST = a.nstages;
-  unsigned long long* full = reinterpret_cast<unsigned long long*>(ring + (size_t)NST * SB);
-  unsigned long long* empty = full + NST;
-  __shared__ int s_abort;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int4 it = a.items[blockIdx.x];
-  if (threadIdx.x == 0) {
-    s_abort = 0;
-    for (int q = 0; q < NST; ++q) {
-      mbar_init(&full[q], 1);
-      mbar_init(&empty[q], ncw);
-    }
-    mbar_fence_init();
-  }
-  for (int i = threadIdx.x; i < NPOL * PG2; i += blockDim.x) acc_s[i] = make_float2(0.f, 0.f);
-  __syncthreads();
-  int nfill = 0;
-  if (warp == ncw) {
-    // ---- producer
-    const unsigned fm = 0xffffffffu;
-    const unsigned rowbytes = (unsigned)prow * sizeof(float2);
-    int seg = 0, cur_plane = -1, why = 1;
-    bool ok = true;
-    const long long ncube = a.v.nrow * (long long)a.v.nchan;
-    auto load = [&](int base, int4& r, float2 (&v)[NPOL]) {
-      const int i = base + lane;
-      if (i < it.z) {
-        r = a.rec[i];
-        if (a.svis) {
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) v[p] = a.svis[(size_t)i * a.npol_total + a.pol0 + p];
-        } else {
-          // the weighted visibilities straight from the cube (random 8-byte
-          // reads, a window ahead of their use, beside a compute-bound kernel)
-          const unsigned nr32 = (unsigned)a.v.nrow;
-          const int chan = (int)((unsigned)r.w / nr32);
-          float pr = 1.f, pi = 0.f;
-          if (!a.v.psf && !a.v.pcf) phasor_of(a.v, (long long)((unsigned)r.w - (unsigned)chan * nr32), chan, &pr, &pi);
-          const float m = a.v.mfs ? a.v.mfs[chan] : 1.f;
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) v[p] = weighted_vis(a.v, r.w, ncube, a.pol0 + p, pr, pi, m);
-        }
-      } else {
-        r = make_int4(0, 0, -1, -1);
-      }
-    };
-    auto acquire = [&](int stage) -> bool {
-      bool okw = true;
-      if (seg >= NST && lane == 0) okw = mbar_wait(&empty[stage], (unsigned)((seg / NST) - 1) & 1u);
-      return __shfl_sync(fm, okw ? 1 : 0, 0) != 0;
-    };
-    int4 r;
-    float2 v[NPOL];
-    load(it.y, r, v);
-    for (int base = it.y; base < it.z && ok; base += 32) {
-      int4 rn;
-      float2 vn[NPOL];
-      load(base + 32, rn, vn);
-      const int nwin = min(32, it.z - base);
-      const int pl = r.z >= 0 ? r.z / os2 : -1;
-      const int plprev = __shfl_up_sync(fm, pl, 1);
-      unsigned heads = __ballot_sync(fm, lane < nwin && (lane == 0 || plprev != pl));
-      while (heads) {
-        const int h = __ffs(heads) - 1;
-        const unsigned rest = heads & (heads - 1);
-        const int h2 = rest ? __ffs(rest) - 1 : nwin;
-        heads = rest;
-        const int stage = seg % NST;
-        if (!acquire(stage)) { ok = false; break; }
-        unsigned char* sp = ring + (size_t)stage * SB;
-        if (lane >= h && lane < h2) {
-          // the sample's decode, done once here for every tap thread: footprint
-          // origin cell, residues (and the preconditioner's conjugate flag),
-          // offset of its oversampling plane in the plane buffer
-          const int cb = (r.x & 0xffff) + Pg * ((r.x >> 16) & 0xffff);
-          const int res = (r.y & 1023) | (((r.y >> 10) & 1023) << 10) | (r.y & (int)0x80000000);
-          reinterpret_cast<int4*>(sp)[lane - h] = make_int4(cb, res, (r.z % os2) * prow, 0);
-          float2* vs = reinterpret_cast<float2*>(sp + kSeg * 16);
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) vs[(lane - h) * NPOL + p] = v[p];
-        }
-        const int plane = __shfl_sync(fm, pl, h);
-        if (lane == 0) {
-          int* hdr = reinterpret_cast<int*>(sp + SB - 16);
-          hdr[0] = h2 - h;
-        }
-        __syncwarp();
-        if (plane != cur_plane) {
-          // the plane buffer is free once every earlier segment is consumed
-          bool okp = true;
-          if (lane == 0) {
-            if (seg >= 1) okp = mbar_wait(&empty[(seg - 1) % NST], (unsigned)((seg - 1) / NST) & 1u);
-            if (okp) {
-              fence_proxy_async_smem();
-              mbar_expect_tx(&full[stage], (unsigned)os2 * rowbytes);
-              for (int f = 0; f < os2; ++f)
-                bulk_g2s(planebuf + (size_t)f * prow, a.cf.pad + ((size_t)plane * os2 + f) * 256, rowbytes,
-                         &full[stage]);
-            }
-          }
-          if (!__shfl_sync(fm, okp ? 1 : 0, 0)) {
-            ok = false;
-            why = 3;
-            break;
-          }
-          cur_plane = plane;
-        } else if (lane == 0) {
-          mbar_arrive(&full[stage]);
-        }
-        ++seg;
-      }
-      r = rn;
-#pragma unroll
-      for (int p = 0; p < NPOL; ++p) v[p] = vn[p];
-    }
-    if (ok) {
-      const int stage = seg % NST;
-      if (acquire(stage)) {
-        if (lane == 0) {
-          reinterpret_cast<int*>(ring + (size_t)stage * SB + SB - 16)[0] = -1;
-          mbar_arrive(&full[stage]);
-        }
-        ++seg;
-      } else {
-        ok = false;
-      }
-    }
-    nfill = seg;
-    if (!ok && lane == 0) {
-      raise_error(a.err, YG_ERR_TIMEOUT, timeout_where(2, why, seg, blockIdx.x));
-      s_abort = 1;
-    }
-  } else {
-    // ---- tap warps, in NG groups of nthr / NG threads, group g accumulating
-    // the polarisations g NPOL / NG ..: thread t of a group owns x residue
-    // t mod 16 and the y residues t / 16 + RY q, q < SL (RY = ceil(Wy / SL))
-    constexpr int NPG = NPOL / NG;
-    const int gsz = nthr / NG;
-    const int grp = threadIdx.x / gsz, tl = threadIdx.x - grp * gsz;
-    const int pofs = grp * NPG;
-    const int RY = (Wy + SL - 1) / SL;
-    const int rx = tl & 15, ry0 = tl >> 4;
-    int rcell[SL];
-    float2 racc[SL][NPG];
-#pragma unroll
-    for (int q = 0; q < SL; ++q) {
-      rcell[q] = Pg * Pg + threadIdx.x;          // this thread's trash cell until the first sample
-#pragma unroll
-      for (int p = 0; p < NPG; ++p) racc[q][p] = make_float2(0.f, 0.f);
-    }
-    const bool live = ry0 < RY;
-    for (int nseg = 0;; ++nseg) {
-      const int stage = nseg % NST;
-      if (!mbar_wait(&full[stage], (unsigned)(nseg / NST) & 1u)) {
-        raise_error(a.err, YG_ERR_TIMEOUT, timeout_where(2, 2, nseg, blockIdx.x));
-        s_abort = 1;
-        break;
-      }
-      const unsigned char* sp = ring + (size_t)stage * SB;
-      const int cnt = *reinterpret_cast<const volatile int*>(sp + SB - 16);
-      if (cnt < 0) break;
-      // the staged records, visibilities and CF plane are never written while
-      // the tile is: restrict lets the next samples' loads pass this one's stores
-      const int4* __restrict__ recs = reinterpret_cast<const int4*>(sp);
-      const float2* __restrict__ vs = reinterpret_cast<const float2*>(sp + kSeg * 16);
-      const float2* __restrict__ pb = planebuf;
-      float2* __restrict__ acc = acc_s;
-      if (live) {
-#pragma unroll 2
-        for (int l = 0; l < cnt; ++l) {
-          const int4 r = recs[l];
-          const int jx = (rx - (r.y & 1023)) & 15;
-          const int my = (r.y >> 10) & 1023;
-          const bool conj = a.v.pcf && r.y < 0;
-          float2 vv[NPG];
-#pragma unroll
-          for (int p = 0; p < NPG; ++p) vv[p] = vs[l * NPOL + pofs + p];
-#pragma unroll
-          for (int q = 0; q < SL; ++q) {
-            const int ry = ry0 + RY * q;
-            if (SL > 1 && ry >= Wy) continue;
-            int jy = ry - my;
-            jy += (jy < 0) ? Wy : 0;
-            float2 c = pb[r.z + jy * 16 + jx];
-            if (conj) c.y = -c.y;
-            const int cell = r.x + jx + Pg * jy;
-            if (cell != rcell[q]) {
-              if (GT) {
-                // the thread owns the cell: its reductions land in program order
-#pragma unroll
-                for (int p = 0; p < NPG; ++p) {
-                  float2* gp = acc + (pofs + p) * PG2 + rcell[q];
-                  atomicAdd(&gp->x, racc[q][p].x);
-                  atomicAdd(&gp->y, racc[q][p].y);
-                  racc[q][p] = make_float2(0.f, 0.f);
-                }
-              } else {
-                float2 g[NPG];
-#pragma unroll
-                for (int p = 0; p < NPG; ++p) g[p] = acc[(pofs + p) * PG2 + rcell[q]];
-#pragma unroll
-                for (int p = 0; p < NPG; ++p) {
-                  g[p].x += racc[q][p].x;
-                  g[p].y += racc[q][p].y;
-                  racc[q][p] = make_float2(0.f, 0.f);
-                }
-#pragma unroll
-                for (int p = 0; p < NPG; ++p) acc[(pofs + p) * PG2 + rcell[q]] = g[p];
-              }
-              rcell[q] = cell;
-            }
-#pragma unroll
-            for (int p = 0; p < NPG; ++p) {
-              racc[q][p].x = fmaf(vv[p].x, c.x, fmaf(-vv[p].y, c.y, racc[q][p].x));
-              racc[q][p].y = fmaf(vv[p].x, c.y, fmaf(vv[p].y, c.x, racc[q][p].y));
-            }
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);
-    }
-#pragma unroll
-    for (int q = 0; q < SL; ++q)
-#pragma unroll
-      for (int p = 0; p < NPG; ++p) {
-        float2* gp = acc_s + (pofs + p) * PG2 + rcell[q];
-        if (GT) {
-          atomicAdd(&gp->x, racc[q][p].x);
-          atomicAdd(&gp->y, racc[q][p].y);
-        } else {
-          float2 g = *gp;
-          g.x += racc[q][p].x;
-          g.y += racc[q][p].y;
-          *gp = g;
-        }
-      }
-  }
-  __syncthreads();
-  if (s_abort) {
-    if (warp == ncw && lane == 0) seg_drain(nfill, NST, full);
-    return;
-  }
-  if (GT) return;   // the tile is already in the scratch slot
-  const int P = a.P, P2 = P * P;
-  float2* out = a.scratch + ((size_t)blockIdx.x * a.npol_total + a.pol0) * P2;
-  for (int i = threadIdx.x; i < NPOL * P2; i += blockDim.x) {
-    const int p = i / P2, c = i % P2;
-    out[i] = acc_s[p * PG2 + (c % P) + Pg * (c / P)];
-  }
-}
-
 // Per sorted sample, once per plan: the footprint origin cell inside the
 // padded tile, its residues mod W and the CF width, the CF index, the sample id.
 // Bit 31 of the second word marks the half of the uv plane where the
@@ -1338,8 +944,6 @@ struct HaloArgs {
   int tile, ntx, nty;
   long long ntiles;
   int smax, P;
-  long long slot_pol;        // scratch elements per polarisation of an item (P^2, or the padded tile)
-  int row;                   // scratch row stride (P, or the padded tile's Pg)
 };
 
 __global__ void k_halo_sum(HaloArgs a) {
@@ -1384,7 +988,7 @@ __global__ void k_halo_sum(HaloArgs a) {
         if (m == 0) continue;
         const int b = a.item_base[nt];
         for (int j = 0; j < m; ++j) {
-          const float2 v = a.scratch[((size_t)(b + j) * a.npol + p) * a.slot_pol + px + (size_t)a.row * py];
+          const float2 v = a.scratch[((size_t)(b + j) * a.npol + p) * P2 + px + (size_t)a.P * py];
           sum.x += v.x;
           sum.y += v.y;
           hit = true;
@@ -2244,7 +1848,7 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
   YG_CUDA_TRY(cudaMemsetAsync(pl.tstart.p, 0, nt * 4, st));
   YG_CUDA_TRY(cudaMemsetAsync(pl.tend.p, 0, nt * 4, st));
   YG_CUDA_TRY(cudaMemsetAsync(pl.nvalid_d.p, 0, 16, st));
-  const int kos2 = a.key_planes ? a.os * a.os : 1;
+  const int kos2 = a.key_planes ? std::abs(a.pl_fs) : 1;
   k_tile_bounds<<<grid_dim(n, 256), 256, 0, st>>>(pl.key.as<unsigned long long>(), n, a.mbits, a.cf.ncf, kos2,
                                                   a.invalid_key, pl.tstart.as<int>(), pl.tend.as<int>(),
                                                   pl.nvalid_d.as<long long>());
@@ -2277,6 +1881,7 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
     YG_COUNT_LAUNCH();
   }
   pl.inv_ready = pl.inv_pos_ready = false;
+  pl.keep_inv = a.keep_inv != 0;
   if (a.need_inv && !a.key_planes) {
     YG_CUDA_TRY(pl.inv.ensure((size_t)n * 4));
     YG_CUDA_TRY(cudaMemsetAsync(pl.inv.p, 0xff, (size_t)n * 4, st));
@@ -2296,7 +1901,7 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
     pl.grid_only = true;
     pl.pos_ready = pl.nvalid > 0;
     pl.pos_mode = 2;
-    pl.os2 = a.os * a.os;
+    pl.pl_fs = a.pl_fs;
   } else if (a.pos_major && pl.nvalid > 0) {
     // a second order of the same records for gridding: tile first as before
     // (the work items stay valid), then the position inside the tile, then
@@ -2304,17 +1909,18 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
     // cells (register accumulation in k_grid)
     const long long nv = pl.nvalid;
     // key_alt and val_alt (free once the records are made) hold the new
-    // keys; the primary keys, read last by k_pos_keys, are the sort's
-    // alternate key buffer; only the alternate values need a buffer of
-    // their own (the primary values stay in use by the passes)
+    // keys; the primary keys and values stay in use (the learned CF's inputs
+    // read the keys), so the sort has alternate buffers of its own
     YG_CUDA_TRY(pl.pos_val2.ensure_headroom(nv * 4));
+    YG_CUDA_TRY(pl.pos_key2.ensure_headroom(nv * 8));
     k_pos_keys<<<grid_dim(nv, 256), 256, 0, st>>>(pl.key.as<unsigned long long>(), nv, a.mbits, a.cf.ncf,
-                                                  a.pos_major, a.os * a.os, pl.key_alt.as<unsigned long long>(),
+                                                  a.pos_major, a.pos_major == 2 ? std::abs(a.pl_fs) : 1,
+                                                  pl.key_alt.as<unsigned long long>(),
                                                   pl.val_alt.as<unsigned int>());
     YG_COUNT_LAUNCH();
     if (sort_pairs_tmp_bytes(nv) > pl.sort_tmp.bytes) YG_CUDA_TRY(pl.sort_tmp.ensure(sort_pairs_tmp_bytes(nv)));
     int alt2 = 0;
-    YG_CUDA_TRY(sort_pairs(pl.key_alt.as<unsigned long long>(), pl.key.as<unsigned long long>(),
+    YG_CUDA_TRY(sort_pairs(pl.key_alt.as<unsigned long long>(), pl.pos_key2.as<unsigned long long>(),
                            pl.val_alt.as<unsigned int>(), pl.pos_val2.as<unsigned int>(), nv, end_bit,
                            pl.sort_tmp.p, pl.sort_tmp.bytes, st, &alt2));
     YG_CUDA_TRY(pl.rec_pos.ensure_headroom((size_t)nv * sizeof(int4)));
@@ -2333,7 +1939,7 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
     YG_CUDA_TRY(cudaGetLastError());
     pl.pos_ready = true;
     pl.pos_mode = a.pos_major;
-    pl.os2 = a.os * a.os;
+    pl.pl_fs = a.pl_fs;
   }
   YG_CUDA_TRY(cudaGetLastError());
   return YG_OK;
@@ -2587,22 +2193,21 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
               cudaEvent_t ev1, int mode, const LearnedCF* lcf) {
   const bool learned = lcf && lcf->w16;
   // mode bits: 16 register accumulation of the row layouts; 32 the
-  // position-major records with taps read through L2 (and register accumulation)
-  // mode 64: the plane-major records with each CF plane's offsets staged in
-  // shared memory (k_grid_pl: 16-wide CFs in exact residue rows)
-  const bool planes = (mode & 64) != 0 && pl.pos_ready && pl.pos_mode == 2 && !learned && cf.wpad == 16 &&
-                      pl.wy > 0 && pl.wy <= 16 && !cf.varsup && v.npol <= 4;
+  // position-major records with taps read through L2 (and register
+  // accumulation); 64, or 0 for the automatic choice, the plane-major records
+  // where the plan has them (k_grid_pl)
+  const bool planes = ((mode & 64) != 0 || (mode & 255) == 0) && pl.pos_ready && pl.pos_mode == 2 && !learned &&
+                      !cf.varsup && v.npol <= 4;
   const bool pos = !planes && (mode & 32) != 0 && pl.pos_ready && pl.pos_mode == 1 && !learned && v.npol <= 4;
   const bool racc = (mode & 16) != 0 || pos;
   if (pl.grid_only && !planes && pl.nitems > 0) return YG_ERR_STATE;   // only the plane-major kernel reads it
-  // mode 128 (with 64): the plane-major kernel's tile in the item's scratch slot
-  const bool gtile = planes && (mode & 128) != 0;
+  if (planes && pl.nitems > 0) {
+    k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, pl.rec_pos.as<int4>(), pl.nvalid, sw, err);
+    YG_COUNT_LAUNCH();
+    YG_CUDA_TRY(cudaGetLastError());
+    return plan_grid_pl(pl, v, cf, grid, nx, ny, nchan_img, scratch, svis, err, st, ev0, ev1);
+  }
   mode &= 15;
-  // plane-major kernel layout: 1 one residue row per thread; 2 the same in two
-  // groups of threads, each accumulating half the polarisations; 3 two rows per thread
-  const int pl_sl = mode == 3 ? 2 : 1;
-  const int pl_ng = (mode == 2 && v.npol >= 2) ? 2 : 1;
-  const int gtile_nthr = planes ? pl_ng * ((16 * ((pl.wy + pl_sl - 1) / pl_sl) + 31) / 32 * 32) : 0;
   if (learned && v.pcf) return YG_ERR_UNSUPPORTED;
   if (pl.nitems == 0) return YG_OK;
   if (!cf.pad || cf.wpad <= 0) return YG_ERR_STATE;
@@ -2611,26 +2216,33 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   GridShape shape = learned ? grid_shape_learned(cf.wpad) : grid_shape_variant(cf.wpad, mode);
   if (pl.wy != cf.wpad) {
     // exact rows: thread t owns x residue t mod 16 and y residue t / 16 < wy
-    if (cf.wpad != 16 || pl.wy > 16 || (!learned && mode > 1 && !planes)) return YG_ERR_UNSUPPORTED;
+    if (cf.wpad != 16 || pl.wy > 16 || (!learned && mode > 1)) return YG_ERR_UNSUPPORTED;
     shape = GridShape{(16 * pl.wy + 31) / 32 * 32, 1, 16};
   }
   if (shape.threads == 0) return YG_ERR_UNSUPPORTED;
-  const size_t per_item = gtile ? (size_t)v.npol * ((size_t)Pg * Pg + gtile_nthr) * sizeof(float2)
-                                : (size_t)v.npol * P * P * sizeof(float2);
+  const size_t per_item = (size_t)v.npol * P * P * sizeof(float2);
   YG_CUDA_TRY(scratch.ensure_headroom(per_item * pl.nitems));
   if (v.npol > 4) return YG_ERR_UNSUPPORTED;
   // the weighted visibilities in the order of the records the kernel reads,
-  // gathered in the cube's order (the plane-major kernel's producer forms its
-  // own); the weight checks and the sums of weights over the sorted records
-  if (!planes) {
-    if (!(pos ? pl.inv_pos_ready : pl.inv_ready)) return YG_ERR_STATE;   // a plan made for degridding only
-    YG_CUDA_TRY(svis.ensure_headroom((size_t)std::max(1ll, pl.nvalid) * v.npol * sizeof(float2)));
-    k_gather_cube<<<grid_dim(pl.nsamples, 256), 256, 0, st>>>(v, pos ? pl.inv_pos.as<int>() : pl.inv.as<int>(),
-                                                             svis.as<float2>());
-    YG_COUNT_LAUNCH();
+  // gathered in the cube's order; the weight checks and the sums of weights
+  // over the sorted records.  A plan made for the plane-major kernel gets the
+  // inverse permutation when a pass first asks for these records.
+  if (!pos && !pl.inv_ready) {
+    Plan& p = const_cast<Plan&>(pl);
+    if (!p.keep_inv) return YG_ERR_STATE;   // a plan made for degridding only
+    YG_CUDA_TRY(p.inv.ensure((size_t)pl.nsamples * 4));
+    YG_CUDA_TRY(cudaMemsetAsync(p.inv.p, 0xff, (size_t)pl.nsamples * 4, st));
+    if (pl.nvalid > 0) {
+      k_inverse<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(pl.rec.as<int4>(), pl.nvalid, p.inv.as<int>());
+      YG_COUNT_LAUNCH();
+    }
+    p.inv_ready = true;
   }
-  k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, planes ? pl.rec_pos.as<int4>() : pl.rec.as<int4>(),
-                                                          pl.nvalid, sw, err);
+  YG_CUDA_TRY(svis.ensure_headroom((size_t)std::max(1ll, pl.nvalid) * v.npol * sizeof(float2)));
+  k_gather_cube<<<grid_dim(pl.nsamples, 256), 256, 0, st>>>(v, pos ? pl.inv_pos.as<int>() : pl.inv.as<int>(),
+                                                           svis.as<float2>());
+  YG_COUNT_LAUNCH();
+  k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, pl.rec.as<int4>(), pl.nvalid, sw, err);
   YG_COUNT_LAUNCH();
   GridKArgs g;
   g.Wy = pl.wy;
@@ -2638,7 +2250,7 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   g.items = pl.items.as<int4>();
   g.val = pl.val.as<unsigned int>();
   g.rec = pos ? pl.rec_pos.as<int4>() : pl.rec.as<int4>();
-  g.svis = planes ? nullptr : svis.as<float2>();
+  g.svis = svis.as<float2>();
   g.pos = pl.pos.as<unsigned int>();
   g.cfi = pl.cfi.as<int>();
   g.v = v;
@@ -2693,60 +2305,6 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
     g.stage_bytes = seg_stage_bytes(g.cfbuf, npa);
     smem = grid_smem_bytes(npa, Pg, g.cfbuf, shape.threads, g.nstages);
   }
-  if (planes) {
-    // k_grid_pl: tile + one plane of every oversampling offset + the ring
-    const int os2 = pl.os2;
-    const int sl = pl_sl, ng = pl_ng, nthr_pl = gtile_nthr;
-    const size_t plane_b = ((size_t)os2 * pl.wy * 16 * sizeof(float2) + 127) & ~(size_t)127;
-    g.rec = pl.rec_pos.as<int4>();
-    g.pps = os2;
-    g.cfbuf = 0;
-    npa = 0;
-    for (int c : {4, 2, 1}) {
-      if (c > v.npol || v.npol % c) continue;
-      const size_t tile_b =
-          gtile ? 0 : ((size_t)c * ((size_t)Pg * Pg + nthr_pl) * sizeof(float2) + 127) & ~(size_t)127;
-      const size_t stage = (size_t)seg_stage_bytes(0, c) + 16;
-      // two CTAs per SM where the tile is in global memory and the plane fits twice
-      const size_t budget = (gtile && plane_b + 2 * stage + 256 <= 113 * 1024) ? 113 * 1024 - 256 : 227 * 1024;
-      if (tile_b + plane_b + 2 * stage <= budget) {
-        npa = c;
-        g.nstages = (int)std::min<size_t>(8, (budget - tile_b - plane_b) / stage);
-        g.stage_bytes = seg_stage_bytes(0, c);
-        smem = tile_b + plane_b + (size_t)g.nstages * stage;
-        break;
-      }
-    }
-    if (npa == 0) return YG_ERR_UNSUPPORTED;
-    if (ev0) cudaEventRecord(ev0, st);
-    for (int pol0 = 0; pol0 < v.npol; pol0 += npa) {
-      g.pol0 = pol0;
-      auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<pl.nitems, nthr_pl + 32, smem, st>>>(g);
-        YG_COUNT_LAUNCH();
-      };
-      const int ngl = npa >= 2 ? ng : 1;
-      if (ngl != ng) return YG_ERR_UNSUPPORTED;
-      switch (npa * 100 + sl * 10 + ngl + (gtile ? 1000 : 0)) {
-        case 111: launch(k_grid_pl<1, 1, 1, false>); break;
-        case 121: launch(k_grid_pl<1, 2, 1, false>); break;
-        case 211: launch(k_grid_pl<2, 1, 1, false>); break;
-        case 212: launch(k_grid_pl<2, 1, 2, false>); break;
-        case 221: launch(k_grid_pl<2, 2, 1, false>); break;
-        case 411: launch(k_grid_pl<4, 1, 1, false>); break;
-        case 412: launch(k_grid_pl<4, 1, 2, false>); break;
-        case 421: launch(k_grid_pl<4, 2, 1, false>); break;
-        case 1111: launch(k_grid_pl<1, 1, 1, true>); break;
-        case 1211: launch(k_grid_pl<2, 1, 1, true>); break;
-        case 1212: launch(k_grid_pl<2, 1, 2, true>); break;
-        case 1411: launch(k_grid_pl<4, 1, 1, true>); break;
-        case 1412: launch(k_grid_pl<4, 1, 2, true>); break;
-        default: return YG_ERR_UNSUPPORTED;
-      }
-      YG_CUDA_TRY(cudaGetLastError());
-    }
-  } else {
   if (ev0) cudaEventRecord(ev0, st);
   for (int pol0 = 0; pol0 < v.npol; pol0 += npa) {
     g.pol0 = pol0;
@@ -2776,7 +2334,6 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
     if (e == cudaErrorInvalidConfiguration) return YG_ERR_UNSUPPORTED;
     if (e != cudaSuccess) return YG_ERR_CUDA;
   }
-  }
   if (ev1) cudaEventRecord(ev1, st);
   HaloArgs h;
   h.item_base = pl.itembase.as<int>();
@@ -2793,8 +2350,6 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   h.ntiles = (long long)pl.ntx * pl.nty;
   h.smax = pl.smax;
   h.P = P;
-  h.slot_pol = gtile ? (long long)Pg * Pg + gtile_nthr : (long long)P * P;
-  h.row = gtile ? Pg : P;
   const long long nblocks = pl.ntiles_total;
   if (nblocks > 0x7fffffffll) return YG_ERR_UNSUPPORTED;
   k_halo_sum<<<(unsigned)nblocks, 256, 0, st>>>(h);

@@ -119,7 +119,9 @@ struct BinArgs {
   int mbits;               // bits of the within-tile Morton code
   int wy;                  // row modulus of the residues in the records (0: the padded CF width)
   int pos_major;           // also build second-order records (rec_pos): 1 position-major, 2 plane-major
+  int pl_fs;               // plane-major order: matrices per CF plane (grid_pl_block)
   int key_planes;          // a plan for gridding only: sort once, by the plane-major key (pos_major 2)
+  int keep_inv;            // the CF-major records may be gridded: their inverse permutation can be built later
   int need_inv;            // build the inverse permutation (the cube-order gather of the CF-major kernels)
   unsigned long long invalid_key;  // one past the largest valid key
   CFView cf;
@@ -147,13 +149,14 @@ struct Plan {
   DevBuf chanmap;               // accessor channel -> image channel of the binned chunk
   DevBuf rec;                   // per sorted sample: cell, residues|w, CF index, sample id (int4)
   DevBuf rec_pos;               // the same records ordered by tile, then position in the tile, then CF
-  DevBuf pos_val2;              // alternate values of the rec_pos sort
+  DevBuf pos_val2, pos_key2;    // alternate values and keys of the rec_pos sort
   DevBuf inv, inv_pos;          // per sample id: its index in rec (rec_pos), -1 off the grid
   bool pos_ready = false;       // rec_pos is built
   bool grid_only = false;       // sorted once, plane-major: rec_pos only (no CF-major records)
   bool inv_ready = false, inv_pos_ready = false;   // inv / inv_pos are built
+  bool keep_inv = false;        // inv may be built when a pass first needs it
   int pos_mode = 0;             // its order: 1 position then CF index; 2 CF plane, position, offset
-  int os2 = 1;                  // oversampling offsets per CF plane
+  int pl_fs = 0;                // plane-major records: grid_pl_block of their CF table
   DevBuf ext;                   // continuous learned CF: per sorted sample (ru, rv, w, 0)
   bool ext_ready = false;
   int mbits = 0, ncf = 0;       // sort-key layout
