@@ -1227,9 +1227,18 @@ void Gridder::prepare_corrections() {
     return;
   }
   const int support = (kind_ == Kind::SphFunc) ? sph_support_ : 3;
+  // they depend on the shape alone: made once for the handle's shape (on the
+  // host: another rounding of one factor would change every image that is
+  // predicted, subtracted and gridded with it in the corners)
+  if (corr_d_.p && corr_nx_ == nx_ && corr_ny_ == ny_) return;
+  const Spheroidal g(M_PI * support, alpha_);
+  const std::vector<double> cx = sph_correction(nx_, g), cy = nx_ == ny_ ? cx : sph_correction(ny_, g);
+  corr_nx_ = corr_ny_ = 0;
   cuda_check(corr_d_.ensure((nx_ + ny_) * sizeof(double)), "alloc");
-  rc_check(grid_correction(Spheroidal(M_PI * support, alpha_).series_tables(), nx_, ny_, corr_d_.as<double>(), stream_),
-           "grid correction");
+  cuda_check(cudaMemcpy(corr_d_.p, cx.data(), nx_ * sizeof(double), cudaMemcpyHostToDevice), "up");
+  cuda_check(cudaMemcpy(corr_d_.as<double>() + nx_, cy.data(), ny_ * sizeof(double), cudaMemcpyHostToDevice), "up");
+  corr_nx_ = nx_;
+  corr_ny_ = ny_;
 }
 
 void Gridder::finalise_grid(float* out, bool out_on_device) {

@@ -191,6 +191,7 @@ class Gridder {
   void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
+  int corr_nx_ = 0, corr_ny_ = 0;      // shape that corr_d_ was made for
   void order_after_legacy_stream();
   std::vector<uint8_t> psf_rows(const Chunk& hc);
 

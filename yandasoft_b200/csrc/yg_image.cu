@@ -1,9 +1,9 @@
 // Image-side steps of the gridders on the GPU: finaliseGrid and
 // initialiseDegrid (askap/gridding/TableVisGridder.cc:1109-1236,1286-1319)
 // and the w-stack variants (askap/gridding/WStackVisGridder.cc:134-171,
-// 216-337).  Transforms are batched cuFFT C2C over all (pol, chan) planes; the
-// centring of both sides costs no pass of its own (k_image_accum,
-// k_image_to_uv), and the grid correction
+// 216-337).  Transforms are batched cuFFT C2C over all (pol, chan) planes; for
+// sides that are powers of two the centring of both sides costs no pass of its
+// own (k_image_accum, k_image_to_uv), and the grid correction
 // (SphFuncVisGridder::correctConvolution) is applied as separable FP64 factors
 // in the same passes.
 #include <cufft.h>
@@ -43,7 +43,11 @@ __device__ __forceinline__ bool wstack_screen(const StackScreen& s, int x, int y
 // B the plain backward FFT of a grid, the centred transform is
 //   (-1)^(x + nx/2 + y + ny/2) B[(x + nx/2) mod nx, (y + ny/2) mod ny],
 // so the grid goes into the FFT as it is (out of place; no checkerboard copy
-// of it) and the roll is this kernel's read index.  One thread per output
+// of it) and the roll is this kernel's read index.  That is so bit for bit
+// where both sides are powers of two (the checkerboard then only exchanges
+// halves of every butterfly); other sides (roll = 0) transform the
+// checkerboard copy, whose rounding the corners of an image would show.  One
+// thread per output
 // pixel walks the planes: the w-stack screen (FP64 square root, sine, cosine)
 // is evaluated once for all of them, and only the centre that is kept is read.
 //   acc (+)= real(B' [* screen]), and for the last grid times cx[x] cy[y].
@@ -51,15 +55,16 @@ __device__ __forceinline__ bool wstack_screen(const StackScreen& s, int x, int y
 // 4096^2 x 4 planes: 698 us for checkerboard copy + accumulation before
 // (20 B more traffic, the screen per plane, 64-bit divisions per pixel).
 __global__ void __launch_bounds__(256) k_image_accum(const float2* __restrict__ f, float* __restrict__ acc, int nx,
-                                                     int ny, int onx, int ony, int nplanes, int first, int last,
-                                                     int use_screen, StackScreen scr, const double* __restrict__ cx,
-                                                     const double* __restrict__ cy) {
+                                                     int ny, int onx, int ony, int nplanes, int roll, int first,
+                                                     int last, int use_screen, StackScreen scr,
+                                                     const double* __restrict__ cx, const double* __restrict__ cy) {
   const int ox = blockIdx.x * blockDim.x + threadIdx.x;
   const int oy = blockIdx.y;
   if (ox >= onx) return;
   const int x = ox + (nx - onx) / 2, y = oy + (ny - ony) / 2;
-  const int bx = x + nx / 2 < nx ? x + nx / 2 : x + nx / 2 - nx;
-  const int by = y + ny / 2 < ny ? y + ny / 2 : y + ny / 2 - ny;
+  const int hx = roll ? nx / 2 : 0, hy = roll ? ny / 2 : 0;
+  const int bx = x + hx < nx ? x + hx : x + hx - nx;
+  const int by = y + hy < ny ? y + hy : y + hy - ny;
   const float s = sgn_out(x, y, nx, ny);
   float cr = 1.f, ci = 0.f;
   const bool inside = use_screen && wstack_screen(scr, x, y, &cr, &ci);
@@ -82,20 +87,22 @@ __global__ void __launch_bounds__(256) k_image_accum(const float2* __restrict__ 
 // Forward side: the plain FFT of
 //   (-1)^(x' + y') a[(x' + nx/2) mod nx, (y' + ny/2) mod ny]
 // is the centred transform of a itself, both checkerboards included, so the
-// grids need no sign pass after the FFT.  a is the image in the centre of the
+// grids need no sign pass after the FFT (roll, powers of two; other sides keep
+// it: k_checkerboard).  a is the image in the centre of the
 // padded plane, corrected, and with w-stacks conj(image * screen) (the screen
 // once per pixel for all planes).  HBM bound: 4 B read, 8 B written per cell;
 // 507 us per grid of 4096^2 x 4 planes before with the sign pass (16 B more).
 __global__ void __launch_bounds__(256) k_image_to_uv(const float* __restrict__ img, float2* __restrict__ out, int inx,
-                                                     int iny, int nx, int ny, int nplanes, int use_screen,
-                                                     StackScreen scr, const double* __restrict__ cx,
+                                                     int iny, int nx, int ny, int nplanes, int roll,
+                                                     int use_screen, StackScreen scr, const double* __restrict__ cx,
                                                      const double* __restrict__ cy, int* __restrict__ any) {
   const int bx = blockIdx.x * blockDim.x + threadIdx.x;
   const int by = blockIdx.y;
   bool seen = false;
   if (bx < nx) {
-    const int x = bx + nx / 2 < nx ? bx + nx / 2 : bx + nx / 2 - nx;
-    const int y = by + ny / 2 < ny ? by + ny / 2 : by + ny / 2 - ny;
+    const int hx = roll ? nx / 2 : 0, hy = roll ? ny / 2 : 0;
+    const int x = bx + hx < nx ? bx + hx : bx + hx - nx;
+    const int y = by + hy < ny ? by + hy : by + hy - ny;
     const int ix = x - (nx - inx) / 2, iy = y - (ny - iny) / 2;
     const bool on = ix >= 0 && iy >= 0 && ix < inx && iy < iny;
     float cr = 1.f, ci = 0.f;
@@ -120,97 +127,20 @@ __global__ void __launch_bounds__(256) k_image_to_uv(const float* __restrict__ i
   if (any && __syncthreads_or(seen) && threadIdx.x == 0) *any = 1;
 }
 
-// Spheroidal function of one nu (Spheroidal::operator(), the same recurrence).
-__device__ double sph_value(const SphSeries& t, double nu) {
-  if (!(fabs(nu) < 1.0)) return 0.0;
-  const double s = sqrt(fmax(0.0, 1.0 - nu * nu));
-  double pmm = sqrt(0.5);
-  for (int k = 0; k < t.m; ++k) pmm = -pmm * t.pmm[k] * s;
-  double sum = t.coeff[0] * pmm;
-  double prev = pmm, cur = nu * sqrt(2.0 * t.m + 3.0) * pmm;
-  for (int q = 0; q < 2 * (t.nterms - 1) - 1; ++q) {
-    const double next = t.a[q] * (nu * cur - t.b[q] * prev);
-    prev = cur;
-    cur = next;
-    if ((q & 1) == 0) sum += t.coeff[q / 2 + 1] * next;
+// out = (-1)^(x + y + odd) in, over the planes (in may be out)
+__global__ void __launch_bounds__(256) k_checkerboard(const float2* in, float2* out, int nx, int ny, int nplanes,
+                                                      int odd) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+  if (x >= nx) return;
+  const float s = sgn_in(x, y + odd);
+  for (int p = 0; p < nplanes; ++p) {
+    const size_t i = x + (size_t)nx * (y + (size_t)ny * p);
+    const float2 v = in[i];
+    out[i] = make_float2(v.x * s, v.y * s);
   }
-  return sum / t.sum0 * pow(1.0 - nu * nu, -t.alpha / 2.0);
 }
 
-// Correction factors of one axis per block: the spheroidal over the axis
-// (single precision, edge interpolated), low-passed to its central 2 * 3 + 1
-// Fourier coefficients, scaled to keep the centre, inverted.  Only those seven
-// coefficients exist after the filter, so they are summed directly (n terms
-// each) and the filtered function is their seven-term series: 14 n instead of
-// two transforms, for any n.  Latency bound: two blocks.  Before, on the host
-// with two uploads: 0.3 ms at 1024^2, and a plain n^2 transform at sizes that
-// are not a power of two (590 ms at 3000^2).
-__global__ void __launch_bounds__(1024) k_grid_correction(const __grid_constant__ SphSeries t, int nx, int ny,
-                                                          double* __restrict__ corr) {
-  __shared__ double part[32][7];
-  __shared__ double coef[7];
-  const int n = blockIdx.x == 0 ? nx : ny;
-  double* d = corr + (blockIdx.x == 0 ? 0 : nx);
-  const int half = n / 2;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < n; i += blockDim.x) d[i] = (double)(float)sph_value(t, fabs((double)(i - half)) / (double)half);
-  __syncthreads();
-  if (tid == 0 && n > 3) {
-    const float e = __fadd_rn(__fmul_rn(3.0f, __fsub_rn((float)d[1], (float)d[2])), (float)d[3]);
-    d[0] = (double)e;
-    if (n % 2 == 1) d[n - 1] = (double)e;
-  }
-  __syncthreads();
-  // sums of v cos(2 pi k j / n), k = 0..3, and v sin, k = 1..3, j = i - half
-  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int i = tid; i < n; i += blockDim.x) {
-    const double v = d[i], x = 2.0 * (double)(i - half) / (double)n;
-    acc[0] += v;
-#pragma unroll
-    for (int k = 1; k <= 3; ++k) {
-      double sn, cs;
-      sincospi(k * x, &sn, &cs);
-      acc[k] += v * cs;
-      acc[3 + k] += v * sn;
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < 7; ++q) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], off);
-    if (lane == 0) part[warp][q] = acc[q];
-  }
-  __syncthreads();
-  if (tid < 7) {
-    double sum = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += part[w][tid];
-    coef[tid] = sum;
-  }
-  const double centre = d[half];
-  __syncthreads();
-  // coefficient k is (coef[|k|], -sign(k) coef[3 + |k|]); indices half + k
-  const int klo = max(-3, -half), khi = min(3, n - 1 - half);
-  double c0r = 0.0, c0i = 0.0;
-  for (int k = klo; k <= khi; ++k) {
-    c0r += coef[abs(k)];
-    if (k != 0) c0i += k > 0 ? -coef[3 + k] : coef[3 - k];
-  }
-  const double c2 = c0r * c0r + c0i * c0i;
-  const double nr = centre * c0r / c2, ni = -centre * c0i / c2;      // centre / filtered centre
-  for (int i = tid; i < n; i += blockDim.x) {
-    const double x = 2.0 * (double)(i - half) / (double)n;
-    double vr = 0.0, vi = 0.0;
-    for (int k = klo; k <= khi; ++k) {
-      double sn, cs;
-      sincospi(k * x, &sn, &cs);
-      const double fr = coef[abs(k)], fi = k == 0 ? 0.0 : (k > 0 ? -coef[3 + k] : coef[3 - k]);
-      vr += fr * cs - fi * sn;
-      vi += fr * sn + fi * cs;
-    }
-    const double v = vr * nr - vi * ni;
-    d[i] = fabs(v) > 1e-10 ? 1.0 / v : 0.0;
-  }
-}
+static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
 
 // vals by value: up to 32 planes per launch
 struct PlaneValues {
@@ -262,12 +192,6 @@ ImageFFT::~ImageFFT() {
   if (plan_ok) cufftDestroy(plan);
 }
 
-int grid_correction(const SphSeries& t, int nx, int ny, double* corr, cudaStream_t st) {
-  k_grid_correction<<<2, 1024, 0, st>>>(t, nx, ny, corr);
-  IM_TRY(cudaGetLastError());
-  return YG_OK;
-}
-
 int fill_planes(float* out, long long npix, const std::vector<float>& vals, cudaStream_t st) {
   for (size_t p0 = 0; p0 < vals.size(); p0 += 32) {
     PlaneValues v{};
@@ -287,13 +211,18 @@ int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny,
   if (rc) return rc;
   const long long total = (long long)nx * ny * nplanes;
   const bool corr = corr_x && corr_y;
+  const bool roll = power_of_two(nx) && power_of_two(ny);
   for (int g = 0; g < ngrids; ++g) {
-    if (cufftExecC2C(f.plan, (cufftComplex*)(grids + (size_t)g * total), (cufftComplex*)f.work.p, CUFFT_INVERSE) !=
-        CUFFT_SUCCESS)
+    const float2* src = grids + (size_t)g * total;
+    if (!roll) {
+      k_checkerboard<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(src, f.work.as<float2>(), nx, ny, nplanes, 0);
+      src = f.work.as<float2>();
+    }
+    if (cufftExecC2C(f.plan, (cufftComplex*)src, (cufftComplex*)f.work.p, CUFFT_INVERSE) != CUFFT_SUCCESS)
       return YG_ERR_CUDA;
     const bool use = screens != nullptr;
     k_image_accum<<<dim3((onx + 255) / 256, ony), 256, 0, st>>>(
-        f.work.as<float2>(), out, nx, ny, onx, ony, nplanes, g == 0, g == ngrids - 1, use,
+        f.work.as<float2>(), out, nx, ny, onx, ony, nplanes, roll, g == 0, g == ngrids - 1, use,
         use ? (*screens)[g] : StackScreen{}, corr ? corr_x : nullptr, corr_y);
   }
   IM_TRY(cudaGetLastError());
@@ -307,13 +236,16 @@ int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, in
   if (rc) return rc;
   const long long total = (long long)nx * ny * nplanes;
   const bool corr = corr_x && corr_y;
+  const bool roll = power_of_two(nx) && power_of_two(ny);
   for (int g = 0; g < ngrids; ++g) {
     float2* dst = grids + (size_t)g * total;
     const bool use = screens != nullptr;
-    k_image_to_uv<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(image, dst, inx, iny, nx, ny, nplanes, use,
+    k_image_to_uv<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(image, dst, inx, iny, nx, ny, nplanes, roll, use,
                                                              use ? (*screens)[g] : StackScreen{},
                                                              corr ? corr_x : nullptr, corr_y, g == 0 ? any : nullptr);
     if (cufftExecC2C(f.plan, (cufftComplex*)dst, (cufftComplex*)dst, CUFFT_FORWARD) != CUFFT_SUCCESS) return YG_ERR_CUDA;
+    if (!roll)
+      k_checkerboard<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(dst, dst, nx, ny, nplanes, nx / 2 + ny / 2);
   }
   IM_TRY(cudaGetLastError());
   return YG_OK;

@@ -5,7 +5,6 @@
 #include <vector>
 
 #include "yg_internal.h"
-#include "yg_spheroidal.h"
 
 namespace yg {
 
@@ -25,10 +24,6 @@ struct ImageFFT {
   int ensure(int nx, int ny, int nplanes, cudaStream_t st);
   ~ImageFFT();
 };
-
-// Correction factors of SphFuncVisGridder::correctConvolution
-// (SphFuncVisGridder.cc:171-248): corr[0, nx) along x, corr[nx, nx + ny) along y.
-int grid_correction(const SphSeries& t, int nx, int ny, double* corr, cudaStream_t st);
 
 // out (onx, ony, nplanes), device: the centre of
 // corr_x corr_y sum_g real(backward FFT(grid_g) [* screen_g]) over (nx, ny)

@@ -10,23 +10,10 @@
 
 namespace yg {
 
-// The Legendre series of a Spheroidal as plain numbers, passed by value to the
-// kernel that evaluates it: P_l^m by the upward recurrence
-// P_l = a[l - m - 2] (x P_{l-1} - b[l - m - 2] P_{l-2}).
-struct SphSeries {
-  static constexpr int kTerms = 16;
-  int m = 0, nterms = 0;
-  double alpha = 0, sum0 = 1;
-  double coeff[kTerms] = {};
-  double pmm[2] = {};                    // P_k^k from P_{k-1}^{k-1}: -pmm[k - 1] sqrt(1 - x^2), k = 1..m
-  double a[2 * kTerms] = {}, b[2 * kTerms] = {};
-};
-
 class Spheroidal {
  public:
   Spheroidal(double c, double alpha, int nterms = 16);
   double operator()(double nu) const;
-  SphSeries series_tables() const;
 
  private:
   double series(double eta) const;
@@ -36,5 +23,9 @@ class Spheroidal {
   std::vector<double> coeffs_;
   double sum0_;
 };
+
+// 1-D filtered correction factors of SphFuncVisGridder::correctConvolution
+// (askap/gridding/SphFuncVisGridder.cc:171-248) for an axis of n pixels.
+std::vector<double> sph_correction(int n, const Spheroidal& grdsf, bool interp = true);
 
 }  // namespace yg
