@@ -1,4 +1,4 @@
-"""k_grid_pl (plane-major gridding) against the oracle at the edges of its
+"""k_grid_pl (plane-major gridding) and k_grid_cf (CF-major) against the oracle at the edges of its
 layouts: CF widths around multiples of a warp's 32 residues, one and several
 parts and groups, staged and unstaged tables, one to four polarisations, tiles
 and work items of odd sizes, and scratch in several batches."""
@@ -110,3 +110,39 @@ def test_scratch_batches():
         out.append((np.stack(gg.grids()), gg.sum_weights()))
     assert rel_l2(out[0][0], out[1][0]) < TOL
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("support,os_,npol,tile,item,diameter,mode", [
+    (3, 4, 1, 0, 0, 600.0, ""), (3, 8, 2, 24, 300, 60.0, "psf"), (4, 8, 4, 40, 5000, 60.0, ""),
+    (6, 8, 4, 32, 700, 600.0, ""), (6, 8, 3, 32, 257, 600.0, "pcf"), (7, 8, 4, 24, 129, 600.0, ""),
+    (8, 4, 2, 56, 100, 600.0, "pcf"), (9, 8, 4, 40, 3000, 60.0, ""), (12, 4, 2, 24, 511, 600.0, ""),
+    (15, 4, 1, 32, 90, 600.0, "psf"), (19, 4, 4, 32, 400, 600.0, ""), (24, 4, 1, 56, 1300, 600.0, ""),
+    (27, 4, 1, 48, 800, 60.0, "pcf"), (30, 4, 2, 32, 2000, 600.0, "")])
+def test_cf_major_same_sums(support, os_, npol, tile, item, diameter, mode):
+    """The default CF-major kernel adds a cell's samples in the order of the
+    padded layout (variant 2: half its threads, the same order), bit for bit;
+    against the oracle within the order of its sums."""
+    import oracle
+    from yandasoft_b200.gridder import Accessor, Axes
+    ds, flag, noise, delay = _inputs(npol, diameter, 200 + support)
+    og, gg = _pair(support, os_)
+    if tile:
+        gg.set_tile(tile)
+    if item:
+        gg.set_item_size(item)
+    kw = {"psf": {"dopsf": True}, "pcf": {"dopcf": True}}.get(mode, {})
+    acc = Accessor(ds.uvw, ds.freq, ds.vis, noise=noise, flag=flag, delay=delay).to_device()
+    out = []
+    for variant in (0, 2):
+        gg.set_grid_variant(variant)
+        gg.initialiseGrid(Axes(CELL, CELL), (NX, NX, npol, 1), **kw)
+        gg.grid(acc)
+        out.append(np.stack(gg.grids()))
+    assert gg.support()[0] == support
+    assert np.array_equal(out[0], out[1])
+    chunk = oracle.Chunk(uvw=ds.uvw, freq=ds.freq, vis=ds.vis, noise=noise, flag=flag, delay=delay)
+    og.initialise_grid(NX, NX, npol, 1, CELL, CELL, **kw)
+    og.init_cf(chunk)
+    _adopt_cf(og, gg)
+    og.grid(chunk)
+    assert rel_l2(out[0], np.stack(og.grids)) < TOL

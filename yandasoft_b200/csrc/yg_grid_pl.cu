@@ -452,6 +452,269 @@ __global__ void __launch_bounds__(NPOL == 1 ? 416 : (SL <= 4 ? 288 : 256), NPOL 
   }
 }
 
+struct GridCfArgs {
+  const int4* items;
+  const int4* rec;           // CF-major records
+  const float2* svis;        // weighted visibilities, [sample][npol]
+  int npol, pcf, pol0;
+  const float2* cf;
+  const long long* cfoff;
+  int W, P;
+  int Wx, nres;              // residue modulus along x (W rounded up to 8), Wx x W residues
+  int nw;                    // tap warps
+  int cf_bytes;              // CFS: one matrix, rounded up to 16 bytes
+  int stage_bytes, nstages, fetch_off;
+  float2* scratch;           // [item] P x P cells x NPOL
+  long long slot;
+  DevError* err;
+};
+
+// GridKernel::grid over the CF-major records, every cell's sum in the order of
+// its samples: the sums of k_grid bit for bit (it adds zero taps besides).  One
+// CTA per work item; thread t of the tap warps owns the residues k = t + 32 nw q
+// of the footprint, rows modulo the exact CF width W and columns, with staged
+// CFs, modulo W rounded up to 8 (k_grid: both up to 16, 1.2 to 5 times the
+// taps), so no two threads touch one cell, and eight lanes of a row always lie
+// on eight different 16-byte banks (modulo W itself a footprint's wrap puts two
+// lanes on one: 35.7 instead of 30.0 ms at W 13, 4 polarisations, 4.4e7
+// samples; unstaged, the latency of the taps hides it and the idle lanes of the
+// rounding cost more: 7.4 against 11.9 ms at W 67 to 73).  The
+// shared-memory tile holds two polarisations of a cell together (a plane of
+// 16-byte cells per pair: neighbouring lanes on neighbouring banks); all slots of a thread are loaded before any is
+// stored.  CFS: a segment is up to 32 samples of one CF matrix, brought into
+// its stage by one bulk copy; otherwise 32 samples of any, the taps through
+// L1 / L2 (matrices too large to stage beside the tile, and oversampling so
+// fine that hardly two samples share one).
+// Bound by shared memory (16 NPOL + 8 bytes per tap) and the latency from one
+// sample's stores to the next one's loads.  Per launch, k_grid with its gather
+// and inverse permutation, and now with k_weigh_cube: W 13, 4.4e7 samples x 4:
+// 42.6 -> 30.5 ms; W 19, 2.1e7 x 4: 70.4 -> 30.8; W 49, 1.6e6 x 1: 6.3 -> 4.6;
+// W 67 to 73, 1.5e6 x 1: 14.1 -> 7.4; W 7, 2.8e6 x 2: 2.5 -> 1.6.
+template <int NPOL, int SL, bool CFS>
+__global__ void __launch_bounds__(544, 1) k_grid_cf(const __grid_constant__ GridCfArgs a) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  float2* tile = reinterpret_cast<float2*>(smem_raw);
+  unsigned char* ring = smem_raw + (((size_t)a.slot * sizeof(float2) + 127) & ~(size_t)127);
+  const int SB = a.stage_bytes, NST = a.nstages;
+  unsigned long long* full = reinterpret_cast<unsigned long long*>(ring + (size_t)NST * SB);
+  unsigned long long* empty = full + NST;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int4 it = a.items[blockIdx.x];
+  __shared__ int s_abort;
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int q = 0; q < NST; ++q) {
+      mbar_init(&full[q], 1);
+      mbar_init(&empty[q], a.nw);
+    }
+    mbar_fence_init();
+  }
+  const int n4 = (int)(a.slot / 2);
+  for (int i = threadIdx.x; i < n4; i += blockDim.x)
+    reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  const int W = a.W;
+  const int rec_at = CFS ? a.cf_bytes : 0, vis_at = rec_at + kSeg * 16;
+  if (warp == a.nw) {
+    // ---- producer (as k_grid_pl's)
+    const unsigned fm = 0xffffffffu;
+    const int Wx = a.Wx;
+    const float rW = __frcp_rn((float)W) * (1.f + 1e-6f), rWx = __frcp_rn((float)Wx) * (1.f + 1e-6f);
+    Fetch<NPOL>& f = *reinterpret_cast<Fetch<NPOL>*>(ring + a.fetch_off);
+    auto fetch_rec = [&](int w) {
+      const int i = it.y + 32 * w + lane;
+      if (i < it.z) copy_async<16>(&f.rec[w % (2 * kAhead)][lane], a.rec + i);
+    };
+    auto fetch = [&](int w) {
+      if (it.y + 32 * w + lane >= it.z) return;
+      const int k = w % kAhead;
+      const int4 r = f.rec[w % (2 * kAhead)][lane];
+      copy_async<8>(&f.off[k][lane], a.cfoff + r.z);
+      const float2* src = a.svis + (size_t)(unsigned)r.w * a.npol + a.pol0;
+      copy_async<NPOL == 1 ? 8 : 16>(&f.vis[k][lane][0], src);
+      if (NPOL == 4) copy_async<16>(&f.vis[k][lane][NPOL / 2], src + 2);
+    };
+    const int nwin_all = (it.z - it.y + 31) / 32;
+    for (int w = 0; w < 2 * kAhead; ++w) fetch_rec(w);
+    copy_commit();
+    copy_wait<0>();
+    for (int w = 0; w < kAhead; ++w) {
+      fetch(w);
+      copy_commit();
+    }
+    int seg = 0;
+    bool ok = true;
+    auto acquire = [&](int stage) -> bool {
+      bool okw = true;
+      if (seg >= NST && lane == 0) okw = mbar_wait(&empty[stage], (unsigned)((seg / NST) - 1) & 1u);
+      return __shfl_sync(fm, okw ? 1 : 0, 0) != 0;
+    };
+    for (int w = 0; w < nwin_all && ok; ++w) {
+      copy_wait<kAhead - 1>();
+      const int nwin = min(32, it.z - it.y - 32 * w), k = w % kAhead;
+      const int4 r = lane < nwin ? f.rec[w % (2 * kAhead)][lane] : make_int4(-1, 0, -1, -1);
+      const long long off = lane < nwin ? f.off[k][lane] : 0;
+      const int px0 = r.x & 0xffff, py0 = (r.x >> 16) & 0xffff;
+      const int zprev = __shfl_up_sync(fm, r.z, 1);
+      unsigned heads = __ballot_sync(fm, lane < nwin && (lane == 0 || (CFS && zprev != r.z)));
+      while (heads) {
+        const int h = __ffs(heads) - 1;
+        const unsigned rest = heads & (heads - 1);
+        const int h2 = rest ? __ffs(rest) - 1 : nwin;
+        heads = rest;
+        const int stage = seg % NST;
+        if (!acquire(stage)) {
+          ok = false;
+          break;
+        }
+        unsigned char* sp = ring + (size_t)stage * SB;
+        if (lane >= h && lane < h2) {
+          reinterpret_cast<int4*>(sp + rec_at)[lane - h] =
+              make_int4(px0 + a.P * py0,
+                        (px0 - Wx * (int)((float)px0 * rWx)) | ((py0 - W * (int)((float)py0 * rW)) << 16),
+                        CFS ? 0 : (int)off, 0);
+          const bool conj = a.pcf && r.y < 0;
+          float4* vs = reinterpret_cast<float4*>(sp + vis_at);
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p) {
+            const float2 x = f.vis[k][lane][p];
+            vs[(lane - h) * NPOL + p] = make_float4(x.x, conj ? -x.x : x.x, x.y, x.y);
+          }
+        }
+        const long long o = __shfl_sync(fm, off, h);
+        if (lane == 0) reinterpret_cast<int*>(sp + SB - 16)[0] = h2 - h;
+        __syncwarp();
+        if (lane == 0) {
+          if (CFS) {
+            fence_proxy_async_smem();
+            mbar_expect_tx(&full[stage], (unsigned)a.cf_bytes);
+            bulk_g2s(sp, a.cf + o, (unsigned)a.cf_bytes, &full[stage]);
+          } else {
+            mbar_arrive(&full[stage]);
+          }
+        }
+        ++seg;
+      }
+      fetch(w + kAhead);
+      fetch_rec(w + 2 * kAhead);
+      copy_commit();
+    }
+    copy_wait<0>();
+    if (ok && acquire(seg % NST)) {
+      if (lane == 0) {
+        reinterpret_cast<int*>(ring + (size_t)(seg % NST) * SB + SB - 16)[0] = -1;
+        mbar_arrive(&full[seg % NST]);
+      }
+    } else if (lane == 0) {
+      raise_error(a.err, YG_ERR_TIMEOUT, timeout_where(1, 1, seg, blockIdx.x));
+      s_abort = 1;
+      // no copy may be in flight when the CTA exits
+      if (CFS)
+        for (int q = 0; q < NST && q < seg; ++q) mbar_wait(&full[q], (unsigned)((seg - q + NST - 1) / NST - 1) & 1u);
+    }
+  } else {
+    // ---- tap warps
+    const int nthr = 32 * a.nw, t = threadIdx.x;
+    const int P2 = a.P * a.P, Wx = a.Wx;
+    int rx[SL], ry[SL];
+    bool live[SL];
+#pragma unroll
+    for (int q = 0; q < SL; ++q) {
+      const int k = q * nthr + t;
+      live[q] = k < a.nres;
+      rx[q] = live[q] ? k % Wx : 0;
+      ry[q] = live[q] ? k / Wx : 0;
+    }
+    for (int seg = 0;; ++seg) {
+      const int stage = seg % NST;
+      if (!mbar_wait(&full[stage], (unsigned)(seg / NST) & 1u)) {
+        if (lane == 0) raise_error(a.err, YG_ERR_TIMEOUT, timeout_where(1, 2, seg, blockIdx.x));
+        s_abort = 1;
+        break;
+      }
+      const unsigned char* sp = ring + (size_t)stage * SB;
+      const int cnt = *reinterpret_cast<const volatile int*>(sp + SB - 16);
+      if (cnt < 0) break;
+      const float2* __restrict__ cfs = reinterpret_cast<const float2*>(sp);
+      const int4* __restrict__ recs = reinterpret_cast<const int4*>(sp + rec_at);
+      const float4* __restrict__ vs = reinterpret_cast<const float4*>(sp + vis_at);
+      float2* __restrict__ g_s = tile;
+      float4* __restrict__ g4 = reinterpret_cast<float4*>(tile);
+#pragma unroll(SL* NPOL <= 8 ? 2 : 1)
+      for (int l = 0; l < cnt; ++l) {
+        const int4 r = recs[l];
+        const int mx = r.y & 0xffff, my = r.y >> 16;
+        float4 vv[NPOL];
+#pragma unroll
+        for (int p = 0; p < NPOL; ++p) vv[p] = vs[l * NPOL + p];
+        float2 c[SL];
+        int cell[SL];
+        bool on[SL];
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          int jx = rx[q] - mx, jy = ry[q] - my;
+          jx += jx < 0 ? Wx : 0;
+          jy += jy < 0 ? W : 0;
+          const int tap = jx + W * jy;
+          on[q] = live[q] && (!CFS || jx < W);
+          if (CFS) {
+            c[q] = make_float2(0.f, 0.f);
+            if (on[q]) c[q] = cfs[tap];
+          } else {
+            c[q] = __ldg(a.cf + r.z + tap);
+          }
+          cell[q] = r.x + jx + a.P * jy;
+        }
+        float2 g[SL][NPOL];
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          if (!on[q]) continue;
+          if (NPOL == 1) {
+            g[q][0] = g_s[cell[q]];
+          } else {
+#pragma unroll
+            for (int p = 0; p < NPOL; p += 2) {
+              const float4 w = g4[cell[q] + p / 2 * P2];
+              g[q][p] = make_float2(w.x, w.y);
+              g[q][(p + 1) % NPOL] = make_float2(w.z, w.w);
+            }
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          const float2 cs = make_float2(-c[q].y, c[q].x);
+#pragma unroll
+          for (int p = 0; p < NPOL; ++p)
+            g[q][p] = fma2(make_float2(vv[p].x, vv[p].y), c[q], fma2(make_float2(vv[p].z, vv[p].w), cs, g[q][p]));
+        }
+#pragma unroll
+        for (int q = 0; q < SL; ++q) {
+          if (!on[q]) continue;
+          if (NPOL == 1) {
+            g_s[cell[q]] = g[q][0];
+          } else {
+#pragma unroll
+            for (int p = 0; p < NPOL; p += 2)
+              g4[cell[q] + p / 2 * P2] =
+                  make_float4(g[q][p].x, g[q][p].y, g[q][(p + 1) % NPOL].x, g[q][(p + 1) % NPOL].y);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[stage]);
+    }
+  }
+  __syncthreads();
+  if (s_abort) return;
+  float4* out = reinterpret_cast<float4*>(a.scratch + (size_t)blockIdx.x * a.slot);
+  const float4* t4 = reinterpret_cast<const float4*>(tile);
+  if (NPOL == 4) {
+    for (int i = threadIdx.x; i < n4; i += blockDim.x) out[i] = t4[(i >> 1) + (i & 1) * a.P * a.P];
+  } else {
+    for (int i = threadIdx.x; i < n4; i += blockDim.x) out[i] = t4[i];
+  }
+}
+
 // grid[cell] += sum over the slots whose padded tile covers the cell, in a
 // fixed order (neighbouring tiles, their items, their groups).  One CTA per
 // (grid plane / channel, tile), one thread per cell for all polarisations (a
@@ -562,6 +825,7 @@ __global__ void __launch_bounds__(256) k_halo_pl(const __grid_constant__ HaloPlA
 // Shared memory of a CTA, and what two CTAs of one SM may each take of it.
 constexpr size_t kSmemOne = 227 * 1024;
 constexpr size_t kSmemTwo = 113 * 1024;
+constexpr size_t kSmemThree = 75 * 1024 - 128;
 
 struct Shape {
   int sl = 0, nw = 0, parts = 1, groups = 1, nstages = 0;
@@ -631,6 +895,51 @@ cudaError_t launch_any(const GridPlArgs& a, const Shape& s, int npol, int nitems
   }
 }
 
+int weigh_cube(const Plan& pl, const VisArgs& v, DevBuf& svis, cudaStream_t st) {
+  if (svis.ensure_headroom((size_t)pl.nsamples * v.npol * sizeof(float2)) != cudaSuccess) return YG_ERR_CUDA;
+  const unsigned blocks = (unsigned)std::max(1ll, std::min((pl.nsamples + 255) / 256, 148ll * 32));
+  switch (v.npol) {
+    case 1: k_weigh_cube<1><<<blocks, 256, 0, st>>>(v, svis.as<float2>()); break;
+    case 2: k_weigh_cube<2><<<blocks, 256, 0, st>>>(v, svis.as<float2>()); break;
+    case 3: k_weigh_cube<3><<<blocks, 256, 0, st>>>(v, svis.as<float2>()); break;
+    default: k_weigh_cube<4><<<blocks, 256, 0, st>>>(v, svis.as<float2>()); break;
+  }
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError() == cudaSuccess ? YG_OK : YG_ERR_CUDA;
+}
+
+HaloPlArgs halo_args(const Plan& pl, const VisArgs& v, float2* grid, int nx, int ny, int nchan_img, int groups,
+                     long long slot) {
+  HaloPlArgs h{};
+  h.item_base = pl.itembase.as<int>();
+  h.nit = pl.nit.as<int>();
+  h.items = pl.items.as<int4>();
+  h.grid = grid;
+  h.nx = nx;
+  h.ny = ny;
+  h.npol = v.npol;
+  h.nchan_img = nchan_img;
+  h.tile = pl.tile;
+  h.ntx = pl.ntx;
+  h.nty = pl.nty;
+  h.ntiles = (long long)pl.ntx * pl.nty;
+  h.smax = pl.smax;
+  h.P = pl.pad;
+  h.groups = groups;
+  h.slot = slot;
+  return h;
+}
+
+int halo_sum(const HaloPlArgs& h, int npa, unsigned nblocks, cudaStream_t st) {
+  switch (npa) {
+    case 1: k_halo_pl<1><<<nblocks, 256, 0, st>>>(h); break;
+    case 2: k_halo_pl<2><<<nblocks, 256, 0, st>>>(h); break;
+    default: k_halo_pl<4><<<nblocks, 256, 0, st>>>(h); break;
+  }
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError() == cudaSuccess ? YG_OK : YG_ERR_CUDA;
+}
+
 // polarisations per pass: the most whose groups fit
 int pols_per_pass(int W, int npol, size_t block) {
   for (int c : {4, 2, 1})
@@ -691,35 +1000,11 @@ int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* gri
   const int batch = (int)std::min<long long>(pl.nitems, std::max<long long>(1184, (long long)(kScratch / per_item)));
   if (scratch.ensure_headroom(per_item * batch) != cudaSuccess) return YG_ERR_CUDA;
   g.scratch = scratch.as<float2>();
-  if (svis.ensure_headroom((size_t)pl.nsamples * v.npol * sizeof(float2)) != cudaSuccess) return YG_ERR_CUDA;
+  int rc = weigh_cube(pl, v, svis, st);
+  if (rc) return rc;
   g.svis = svis.as<float2>();
-  const unsigned wblocks = (unsigned)std::max(1ll, std::min((pl.nsamples + 255) / 256, 148ll * 32));
-  switch (v.npol) {
-    case 1: k_weigh_cube<1><<<wblocks, 256, 0, st>>>(v, svis.as<float2>()); break;
-    case 2: k_weigh_cube<2><<<wblocks, 256, 0, st>>>(v, svis.as<float2>()); break;
-    case 3: k_weigh_cube<3><<<wblocks, 256, 0, st>>>(v, svis.as<float2>()); break;
-    default: k_weigh_cube<4><<<wblocks, 256, 0, st>>>(v, svis.as<float2>()); break;
-  }
-  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  if (cudaGetLastError() != cudaSuccess) return YG_ERR_CUDA;
-  HaloPlArgs h;
-  h.item_base = pl.itembase.as<int>();
-  h.nit = pl.nit.as<int>();
-  h.items = g.items;
+  HaloPlArgs h = halo_args(pl, v, grid, nx, ny, nchan_img, s.groups, g.slot);
   h.scratch = g.scratch;
-  h.grid = grid;
-  h.nx = nx;
-  h.ny = ny;
-  h.npol = v.npol;
-  h.nchan_img = nchan_img;
-  h.tile = pl.tile;
-  h.ntx = pl.ntx;
-  h.nty = pl.nty;
-  h.ntiles = (long long)pl.ntx * pl.nty;
-  h.smax = pl.smax;
-  h.P = P;
-  h.groups = s.groups;
-  h.slot = g.slot;
   if (pl.ntiles_total > 0x7fffffffll) return YG_ERR_UNSUPPORTED;
   const unsigned nblocks = (unsigned)pl.ntiles_total;
   if (ev0) cudaEventRecord(ev0, st);
@@ -736,14 +1021,151 @@ int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* gri
       h.pol0 = pol0;
       h.item0 = i0;
       h.item1 = i0 + n;
-      switch (npa) {
-        case 1: k_halo_pl<1><<<nblocks, 256, 0, st>>>(h); break;
-        case 2: k_halo_pl<2><<<nblocks, 256, 0, st>>>(h); break;
-        default: k_halo_pl<4><<<nblocks, 256, 0, st>>>(h); break;
-      }
-      g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-      if (cudaGetLastError() != cudaSuccess) return YG_ERR_CUDA;
+      rc = halo_sum(h, npa, nblocks, st);
+      if (rc) return rc;
     }
+  }
+  return YG_OK;
+}
+
+namespace {
+
+struct CfShape {
+  int npa = 0, sl = 0, nw = 0, nstages = 0, stage = 0;
+  bool cfs = false;
+  size_t smem = 0;
+};
+
+int cf_stage_bytes(int cf_b, int npa) { return (cf_b + kSeg * 16 + kSeg * npa * 16 + 16 + 127) / 128 * 128; }
+
+// Slots per thread and warps for the residues: two slots share a sample's
+// record and visibilities (W 13: 30.0 ms with two, 31.0 with one, 34.5 with
+// three; W 19: 30.6 / 32.9 / 35.9), one where that leaves fewer than three
+// warps (W 7: 1.6 / 1.9 ms), more where the warps would not fit.
+bool cf_threads(int nres, int npa, int ctas, CfShape* s) {
+  static const int cands[5] = {1, 2, 4, 8, 12};
+  const int wslots = (nres + 31) / 32;
+  for (int sl : cands) {
+    if ((npa >= 2 && sl > 4) || (sl == 1 && wslots > 4)) continue;
+    const int nw = (wslots + sl - 1) / sl;
+    if (nw > 16 || nw * ctas > 48) continue;
+    s->sl = sl;
+    s->nw = nw;
+    return true;
+  }
+  return false;
+}
+
+// As many polarisations per pass as fit at all (W 19: four with one CTA per SM
+// 30.6 ms, two passes of two with two CTAs 35.8), then staged before unstaged
+// CFs (W 49: 4.6 against 5.0 ms), then as many CTAs per SM as fit.  `few`
+// (oversampling above 8): unstaged, hardly two samples share a matrix (W 7:
+// 1.6 against 3.8 ms).
+CfShape cf_shape(int W, int P, int npol, bool few) {
+  const int cf_b = (W * W * 8 + 15) / 16 * 16;
+  for (int npa : {4, 2, 1}) {
+    if (npol % npa) continue;
+    for (int mode = 0; mode < 6; ++mode) {
+      const bool cfs = mode < 3;
+      if (few && cfs) continue;
+      const int ctas = 3 - mode % 3;
+      const size_t budget = ctas == 3 ? kSmemThree : (ctas == 2 ? kSmemTwo : kSmemOne);
+      CfShape s;
+      s.npa = npa;
+      s.cfs = cfs;
+      s.stage = cf_stage_bytes(cfs ? cf_b : 0, npa);
+      const size_t slot = (((size_t)P * P * npa + 1) & ~(size_t)1) * sizeof(float2);
+      const size_t fixed = slot + 448 + fetch_bytes(npa);   // (with the static shared memory)
+      const int want = cfs && cf_b > 8192 ? 2 : 4;
+      if (fixed + want * (size_t)(s.stage + 16) > budget) continue;
+      if (!cf_threads((cfs ? (W + 7) / 8 * 8 : W) * W, npa, ctas, &s)) continue;
+      s.nstages = (int)std::min<size_t>(8, (budget - fixed) / (s.stage + 16));
+      s.smem = fixed + s.nstages * (size_t)(s.stage + 16);
+      return s;
+    }
+  }
+  return CfShape{};
+}
+
+template <int NPOL, int SL, bool CFS>
+cudaError_t launch_cf(const GridCfArgs& a, const CfShape& s, int nitems, cudaStream_t st) {
+  auto k = k_grid_cf<NPOL, SL, CFS>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  if (e != cudaSuccess) return e;
+  k<<<nitems, 32 * (s.nw + 1), s.smem, st>>>(a);
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
+
+template <bool CFS>
+cudaError_t launch_cf_any(const GridCfArgs& a, const CfShape& s, int nitems, cudaStream_t st) {
+  switch (s.npa * 100 + s.sl) {
+    case 101: return launch_cf<1, 1, CFS>(a, s, nitems, st);
+    case 102: return launch_cf<1, 2, CFS>(a, s, nitems, st);
+    case 104: return launch_cf<1, 4, CFS>(a, s, nitems, st);
+    case 108: return launch_cf<1, 8, CFS>(a, s, nitems, st);
+    case 112: return launch_cf<1, 12, CFS>(a, s, nitems, st);
+    case 201: return launch_cf<2, 1, CFS>(a, s, nitems, st);
+    case 202: return launch_cf<2, 2, CFS>(a, s, nitems, st);
+    case 204: return launch_cf<2, 4, CFS>(a, s, nitems, st);
+    case 401: return launch_cf<4, 1, CFS>(a, s, nitems, st);
+    case 402: return launch_cf<4, 2, CFS>(a, s, nitems, st);
+    case 404: return launch_cf<4, 4, CFS>(a, s, nitems, st);
+    default: return cudaErrorInvalidConfiguration;
+  }
+}
+
+}  // namespace
+
+bool grid_cf_takes(const CFView& cf, int P, int npol, int os) {
+  return !cf.varsup && cf.maxsize > 0 && (cf.maxsize & 1) && cf.maxsize <= 1023 && npol <= 4 &&
+         (long long)cf.ncf * (cf.maxsize * cf.maxsize + 1) <= 0x7fffffffll && cf_shape(cf.maxsize, P, npol, os > 8).npa;
+}
+
+int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
+                 int os, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
+                 cudaEvent_t ev1) {
+  const int W = cf.maxsize, P = pl.pad;
+  const CfShape s = cf_shape(W, P, v.npol, os > 8);
+  if (!s.npa) return YG_ERR_UNSUPPORTED;
+  GridCfArgs g;
+  g.items = pl.items.as<int4>();
+  g.rec = pl.rec.as<int4>();
+  g.npol = v.npol;
+  g.pcf = v.pcf;
+  g.cf = cf.data;
+  g.cfoff = cf.off;
+  g.W = W;
+  g.Wx = s.cfs ? (W + 7) / 8 * 8 : W;
+  g.nres = g.Wx * W;
+  g.P = P;
+  g.nw = s.nw;
+  g.cf_bytes = (W * W * 8 + 15) / 16 * 16;
+  g.stage_bytes = s.stage;
+  g.nstages = s.nstages;
+  g.fetch_off = (s.nstages * (s.stage + 16) + 15) & ~15;
+  g.slot = ((long long)P * P * s.npa + 1) & ~1ll;
+  g.err = err;
+  if (scratch.ensure_headroom((size_t)pl.nitems * g.slot * sizeof(float2)) != cudaSuccess) return YG_ERR_CUDA;
+  g.scratch = scratch.as<float2>();
+  int rc = weigh_cube(pl, v, svis, st);
+  if (rc) return rc;
+  g.svis = svis.as<float2>();
+  HaloPlArgs h = halo_args(pl, v, grid, nx, ny, nchan_img, 1, g.slot);
+  h.scratch = g.scratch;
+  if (pl.ntiles_total > 0x7fffffffll) return YG_ERR_UNSUPPORTED;
+  if (ev0) cudaEventRecord(ev0, st);
+  for (int pol0 = 0; pol0 < v.npol; pol0 += s.npa) {
+    g.pol0 = pol0;
+    const cudaError_t e = s.cfs ? launch_cf_any<true>(g, s, pl.nitems, st) : launch_cf_any<false>(g, s, pl.nitems, st);
+    if (e == cudaErrorInvalidConfiguration) return YG_ERR_UNSUPPORTED;
+    if (e != cudaSuccess) return YG_ERR_CUDA;
+    if (ev1 && pol0 + s.npa >= v.npol) cudaEventRecord(ev1, st);
+    h.pol0 = pol0;
+    h.item0 = 0;
+    h.item1 = pl.nitems;
+    rc = halo_sum(h, s.npa, (unsigned)pl.ntiles_total, st);
+    if (rc) return rc;
   }
   return YG_OK;
 }

@@ -1,4 +1,4 @@
-// Plane-major gridding (k_grid_pl).
+// Gridding over plane-major (k_grid_pl) and CF-major records (k_grid_cf).
 #pragma once
 #include "yg_internal.h"
 
@@ -13,5 +13,12 @@ int grid_pl_block(const CFView& cf, int os, int cf_mode, int npol);
 // Grids the plane-major records of a plan (pl.rec_pos, pl.pl_fs).
 int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
                  DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1);
+
+// CF-major gridding with exact residue widths (k_grid_cf): whether it takes the
+// table at this padded tile side, and a pass over the plan's CF-major records.
+bool grid_cf_takes(const CFView& cf, int P, int npol, int os);
+int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
+                 int os, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
+                 cudaEvent_t ev1);
 
 }  // namespace yg

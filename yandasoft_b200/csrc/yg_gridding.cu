@@ -18,6 +18,8 @@
 //                  the cells of a fixed residue class (x mod W, y mod W), so no
 //                  two threads ever touch the same cell (no atomics); its
 //                  weighted visibilities come from k_gather_cube.
+//   k_grid_cf      (yg_grid_pl.cu) the same sums with exact CF widths: the
+//                  default for CF-major records.
 //   k_grid_pl      (yg_grid_pl.cu) over plane-major records, running sums in
 //                  registers.
 //   k_halo_sum     each output tile adds, in a fixed order, the overlapping
@@ -2206,6 +2208,16 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
     YG_COUNT_LAUNCH();
     YG_CUDA_TRY(cudaGetLastError());
     return plan_grid_pl(pl, v, cf, grid, nx, ny, nchan_img, scratch, svis, err, st, ev0, ev1);
+  }
+  // the default CF-major layout: k_grid_cf (the same sums) where it takes the
+  // table; k_grid serves tables of several sizes, the learned CF and the
+  // layouts that are asked for
+  if (!learned && !pl.grid_only && (mode & 255) <= 1 && pl.nitems > 0 && cf.data && pl.keep_inv &&
+      grid_cf_takes(cf, pl.pad, v.npol, sw.os)) {
+    k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, pl.rec.as<int4>(), pl.nvalid, sw, err);
+    YG_COUNT_LAUNCH();
+    YG_CUDA_TRY(cudaGetLastError());
+    return plan_grid_cf(pl, v, cf, grid, nx, ny, nchan_img, sw.os, scratch, svis, err, st, ev0, ev1);
   }
   mode &= 15;
   if (learned && v.pcf) return YG_ERR_UNSUPPORTED;
