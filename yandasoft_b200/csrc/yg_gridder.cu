@@ -828,7 +828,7 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   a.pl_fs = planes && cf_form_ == 0 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
   a.pos_major = a.pl_fs != 0 ? 2 : ((variant & 32) && !(variant & 64) ? 1 : 0);
   a.key_planes = 0;
-  a.need_inv = a.keep_inv = 1;
+  a.keep_inv = 1;
   a.ntx = (nx_ + a.tile - 1) / a.tile;
   a.nty = (ny_ + a.tile - 1) / a.tile;
   int mb = 0;
@@ -898,7 +898,6 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // a gridding-only plan for the plane-major kernel sorts once, by its key
   a.key_planes = (use == PLAN_GRID && a.pos_major == 2) ? 1 : 0;
   a.keep_inv = use != PLAN_DEGRID ? 1 : 0;
-  a.need_inv = (use != PLAN_DEGRID && a.pos_major != 2) ? 1 : 0;
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;

@@ -1884,15 +1884,6 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
   }
   pl.inv_ready = pl.inv_pos_ready = false;
   pl.keep_inv = a.keep_inv != 0;
-  if (a.need_inv && !a.key_planes) {
-    YG_CUDA_TRY(pl.inv.ensure((size_t)n * 4));
-    YG_CUDA_TRY(cudaMemsetAsync(pl.inv.p, 0xff, (size_t)n * 4, st));
-    if (pl.nvalid > 0) {
-      k_inverse<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(pl.rec.as<int4>(), pl.nvalid, pl.inv.as<int>());
-      YG_COUNT_LAUNCH();
-    }
-    pl.inv_ready = true;
-  }
   pl.pos_ready = false;
   pl.grid_only = false;
   if (a.key_planes) {
@@ -2237,8 +2228,8 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   if (v.npol > 4) return YG_ERR_UNSUPPORTED;
   // the weighted visibilities in the order of the records the kernel reads,
   // gathered in the cube's order; the weight checks and the sums of weights
-  // over the sorted records.  A plan made for the plane-major kernel gets the
-  // inverse permutation when a pass first asks for these records.
+  // over the sorted records.  The inverse permutation is built when a pass
+  // first asks for it (k_grid_cf and k_grid_pl need none).
   if (!pos && !pl.inv_ready) {
     Plan& p = const_cast<Plan&>(pl);
     if (!p.keep_inv) return YG_ERR_STATE;   // a plan made for degridding only

@@ -122,7 +122,6 @@ struct BinArgs {
   int pl_fs;               // plane-major order: matrices per CF plane (grid_pl_block)
   int key_planes;          // a plan for gridding only: sort once, by the plane-major key (pos_major 2)
   int keep_inv;            // the CF-major records may be gridded: their inverse permutation can be built later
-  int need_inv;            // build the inverse permutation (the cube-order gather of the CF-major kernels)
   unsigned long long invalid_key;  // one past the largest valid key
   CFView cf;
 };
