@@ -590,9 +590,10 @@ def roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak,
 # polarisation x padded-tile cell, from single-kernel ncu captures of a small
 # case of config 1 (k_grid: the sorted records and visibilities read per
 # sample, the padded tiles written per item)
-# (k_grid_pl: records and the cube's visibility sectors read per sample, the
-# item's global tile reduced and read back per cell)
-TRAFFIC_RATES = {"k_grid": (48.9, 0.84 * 8), "k_grid_pl": (303.0, 26.6)}
+# (k_grid_pl: a record and the weighted visibilities' sector per sample, the
+# rest of the capture apportioned to the cells of the items' slots, cleared and
+# reduced into)
+TRAFFIC_RATES = {"k_grid": (48.9, 0.84 * 8), "k_grid_pl": (48.0, 51.2)}
 
 
 def kgrid_traffic(info, support, npol, name="k_grid"):
@@ -695,7 +696,7 @@ def run_b200(args, w):
     taps = (2 * support + 1) ** 2
     hbm_peak, peak_kind = peaks()
     sm_hz = (clk.summary().get("sm_mhz") or 1965.0) * 1e6
-    variant = args.variant or ((tune or {}).get("variant") or 0)
+    variant = args.variant or ((tune or {}).get("variant") or 0)   # 0: the CF-major default
     roof = roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak, peak_kind, sm_hz,
                     gg.cf_bytes(), kernel_names(variant, support))
     line = {
