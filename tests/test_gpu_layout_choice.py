@@ -1,0 +1,54 @@
+"""Which record order and grid kernel a pass takes: the handle's own choice
+(set_grid_variant, the autotuner, or the automatic choice of its gridder kind),
+never what a plan or another handle happens to bring along."""
+import math
+
+import numpy as np
+import pytest
+
+from parity_helpers import make_pair
+
+pytestmark = pytest.mark.gpu
+
+ARCSEC = math.pi / (180 * 3600)
+CELL = 40.0 * ARCSEC
+NX = 512
+
+
+def _data(npol, seed, diameter=600.0):
+    from yandasoft_b200 import simulate
+    return simulate.make_dataset(duration_s=80.0, nchan=3, npol=npol, seed=seed, diameter_m=diameter)
+
+
+def _wproject(support, os_=8, **more):
+    params = {"wmax": 6000.0, "nwplanes": 5, "oversample": os_, "maxsupport": 1024, "limitsupport": support, **more}
+    return make_pair("WProject", params)[1]
+
+
+def _grid(g, npol, run):
+    from yandasoft_b200.gridder import Axes
+    g.initialiseGrid(Axes(CELL, CELL), (NX, NX, npol, 1))
+    run(g)
+    return np.stack(g.grids())
+
+
+@pytest.mark.parametrize("support,npol", [(3, 2), (6, 4), (19, 1)])
+def test_plan_does_not_choose_the_order(support, npol):
+    """A WProject plan made under variant 64 holds both record orders; under
+    the automatic choice it grids CF-major, the same bits as a plan made
+    without, through this handle and through another of the same parset."""
+    from yandasoft_b200.gridder import Accessor, Axes
+    ds = _data(npol, 300 + support)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    want = _grid(_wproject(support), npol, lambda g: g.grid(acc))
+    assert np.abs(want).max() > 0
+    g = _wproject(support)
+    g.set_grid_variant(64)
+    g.initialiseGrid(Axes(CELL, CELL), (NX, NX, npol, 1))
+    plan = g.plan(acc)
+    planes = _grid(g, npol, lambda g: g.grid_plan(plan, acc))
+    assert not np.array_equal(planes, want)              # the other order rounds differently
+    for variant in (0, 1):
+        g.set_grid_variant(variant)
+        assert np.array_equal(_grid(g, npol, lambda g: g.grid_plan(plan, acc)), want)
+    assert np.array_equal(_grid(_wproject(support), npol, lambda g: g.grid_plan(plan, acc)), want)

@@ -774,6 +774,31 @@ int Gridder::grid_variant() const {
   return 0;
 }
 
+int Gridder::cf_mode() const {
+  switch (kind_) {
+    case Kind::WProject: return CF_MODE_WPLANE;
+    case Kind::AWProject: return CF_MODE_AW;
+    case Kind::WStackWProject: return CF_MODE_WSTACK_WPROJ;
+    default: return CF_MODE_SINGLE;
+  }
+}
+
+// grid_variant() with the automatic choice made: plane-major records (64) for
+// AWProject where the plane-major kernel takes the CF table, CF-major (1)
+// otherwise.  The other gridders' images are divided by the spheroidal, whose
+// factors of 10^4 in the corners turn the rounding of another order of a
+// cell's sum into 1e-4 of the image: their automatic choice keeps the CF-major
+// order, so that an image stays what it was bit for bit, and the plane-major
+// order is theirs to ask for or tune to.  Plans are made by this choice and
+// passes run by it: the records that a plan happens to hold decide nothing.
+int Gridder::grid_layout() const {
+  const int v = grid_variant();
+  if ((v & 255) != 0) return v;
+  const bool planes = kind_ == Kind::AWProject && !aw_taper_ && cf_form_ == 0 &&
+                      grid_pl_block(cf_.view(), os_, cf_mode(), npol_) != 0;
+  return v | (planes ? 64 : 1);
+}
+
 int Gridder::tile_for(int smax, int npol) const {
   if (tile_override_ > 0) return tile_override_;
   TuneChoice c;
@@ -799,13 +824,9 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   a.ny = ny_;
   a.ws = ws_;
   a.ws_stack = ws_stack_;
-  switch (kind_) {
-    case Kind::SphFunc: a.cf_mode = CF_MODE_SINGLE; a.grid_mode = GRID_MODE_SINGLE; break;
-    case Kind::WStack: a.cf_mode = CF_MODE_SINGLE; a.grid_mode = GRID_MODE_WPLANE; break;
-    case Kind::WProject: a.cf_mode = CF_MODE_WPLANE; a.grid_mode = GRID_MODE_SINGLE; break;
-    case Kind::AWProject: a.cf_mode = CF_MODE_AW; a.grid_mode = GRID_MODE_SINGLE; break;
-    case Kind::WStackWProject: a.cf_mode = CF_MODE_WSTACK_WPROJ; a.grid_mode = GRID_MODE_STACK; break;
-  }
+  a.cf_mode = cf_mode();
+  a.grid_mode = kind_ == Kind::WStack ? GRID_MODE_WPLANE
+                                      : (kind_ == Kind::WStackWProject ? GRID_MODE_STACK : GRID_MODE_SINGLE);
   a.aw_nchan = aw_nchan_ > 0 ? aw_nchan_ : 1;
   a.aw_maxfeeds = maxfeeds_;
   a.aw_field = aw_current_field_;
@@ -816,16 +837,10 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   // 16-wide CFs grid with residue rows modulo their real width (exact rows)
   // unless a layout of several slots per thread was asked for
   const int wpad16 = ((2 * smax + 1) + 15) / 16 * 16;
-  const int variant = grid_variant();
+  const int variant = grid_layout();
   a.wy = (wpad16 == 16 && ((variant & 15) <= 1 || (variant & 64)) && exact_rows_) ? 2 * smax + 1 : 0;
-  // Records for the plane-major kernel where it takes the table: asked for by
-  // bit 64, or the automatic choice for AWProject.  The other gridders' images
-  // are divided by the spheroidal, whose factors of 10^4 in the corners turn
-  // the rounding of another order of a cell's sum into 1e-4 of the image: their
-  // automatic choice keeps the CF-major order, so that an image stays what it
-  // was bit for bit, and the plane-major order is theirs to ask for or tune to.
-  const bool planes = (variant & 64) || ((variant & 255) == 0 && kind_ == Kind::AWProject && !aw_taper_);
-  a.pl_fs = planes && cf_form_ == 0 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
+  // records for the plane-major kernel where it takes the table
+  a.pl_fs = (variant & 64) && cf_form_ == 0 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
   a.pos_major = a.pl_fs != 0 ? 2 : ((variant & 32) && !(variant & 64) ? 1 : 0);
   a.key_planes = 0;
   a.keep_inv = 1;
@@ -1104,7 +1119,7 @@ void Gridder::grid_enqueue(const Chunk& dc, const Plan& pl, const float* mfs, cu
                     nsumw_rows_, nchan_};
   const LearnedCF lcf = learned_view_for(dc, const_cast<Plan&>(pl));
   rc_check(plan_grid(pl, v, cf_.view(), grids_.as<float2>(), nx_, ny_, nchan_, sw, scratch_, svis_,
-                     err_.as<DevError>(), st, k0, k1, grid_variant(), cf_form_ != 0 ? &lcf : nullptr),
+                     err_.as<DevError>(), st, k0, k1, grid_layout(), cf_form_ != 0 ? &lcf : nullptr),
            "gridding");
   rc_check(plan_grid_carry(const_cast<Plan&>(pl), v, carry_.as<float2>(), st), "carry");
 }

@@ -155,6 +155,7 @@ class Gridder {
   void set_grid_mode(int m) { grid_mode_ = m; }
   int tile_for(int smax, int npol) const;
   int grid_variant() const;
+  int grid_layout() const;
   int items_vmax() const { return vmax_; }
   void set_vmax(int v) { vmax_ = v; }
   void sync();
@@ -189,6 +190,7 @@ class Gridder {
   void upload_chunk(const Chunk& c, Chunk& dc, bool need_vis, bool vis_writable);
   std::vector<int> chan_map(const double* freq_host, int nchan) const;
   void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
+  int cf_mode() const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
   int corr_nx_ = 0, corr_ny_ = 0;      // shape that corr_d_ was made for

@@ -2185,11 +2185,11 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
               const SumwArgs& sw, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
               cudaEvent_t ev1, int mode, const LearnedCF* lcf) {
   const bool learned = lcf && lcf->w16;
-  // mode bits: 16 register accumulation of the row layouts; 32 the
-  // position-major records with taps read through L2 (and register
-  // accumulation); 64, or 0 for the automatic choice, the plane-major records
-  // where the plan has them (k_grid_pl)
-  const bool planes = ((mode & 64) != 0 || (mode & 255) == 0) && pl.pos_ready && pl.pos_mode == 2 && !learned &&
+  // mode bits (Gridder::grid_layout): 16 register accumulation of the row
+  // layouts; 32 the position-major records with taps read through L2 (and
+  // register accumulation); 64 the plane-major records where the plan has them
+  // (k_grid_pl), which are all that a gridding-only plan of that order holds
+  const bool planes = ((mode & 64) != 0 || pl.grid_only) && pl.pos_ready && pl.pos_mode == 2 && !learned &&
                       !cf.varsup && v.npol <= 4;
   const bool pos = !planes && (mode & 32) != 0 && pl.pos_ready && pl.pos_mode == 1 && !learned && v.npol <= 4;
   const bool racc = (mode & 16) != 0 || pos;
@@ -2203,7 +2203,7 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   // the default CF-major layout: k_grid_cf (the same sums) where it takes the
   // table; k_grid serves tables of several sizes, the learned CF and the
   // layouts that are asked for
-  if (!learned && !pl.grid_only && (mode & 255) <= 1 && pl.nitems > 0 && cf.data && pl.keep_inv &&
+  if (!learned && !pl.grid_only && ((mode & 255) <= 1 || (mode & 255) == 64) && pl.nitems > 0 && cf.data && pl.keep_inv &&
       grid_cf_takes(cf, pl.pad, v.npol, sw.os)) {
     k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, pl.rec.as<int4>(), pl.nvalid, sw, err);
     YG_COUNT_LAUNCH();
