@@ -303,9 +303,13 @@ void yg_cycle_destroy(yg_cycle* c);
 /* ---- autotuner ----
  * No counterpart in the reference.  Times a degrid + grid pass over a
  * device-resident chunk for up to max_trials candidates of (uv tile side,
- * samples per work item, k_grid thread layout) and keeps the fastest for this
- * handle and, process-wide, for every later handle whose CFs have the same
- * padded width and polarisation count.  The handle must be initialised
+ * samples per work item, record order and thread layout of yg_set_grid_variant)
+ * and keeps the fastest for this handle and, process-wide, for every later
+ * handle of the same gridder, oversampling, correction (AWProject with or
+ * without spheroidaltaper), padded CF width and polarisation count.  The
+ * choice may change the order of a cell's sum: images of the corrected
+ * gridders then move by about 1e-4 in their corners, where the correction
+ * amplifies rounding by 10^4.  The handle must be initialised
  * (yg_initialise_grid or yg_initialise_degrid); its grids hold extra passes
  * afterwards, so re-initialise before real use. */
 typedef struct {

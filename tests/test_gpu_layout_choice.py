@@ -52,3 +52,31 @@ def test_plan_does_not_choose_the_order(support, npol):
         g.set_grid_variant(variant)
         assert np.array_equal(_grid(g, npol, lambda g: g.grid_plan(plan, acc)), want)
     assert np.array_equal(_grid(_wproject(support), npol, lambda g: g.grid_plan(plan, acc)), want)
+
+
+@pytest.mark.parametrize("kind,os_", [("AWProject", 4), ("AWProject", 8), ("WProject", 4), ("SphFunc", 8)])
+def test_tuning_serves_its_own_class(kind, os_):
+    """What the autotuner keeps for one gridder kind and oversampling says
+    nothing of another's kernels: a fresh WProject handle of the same padded CF
+    width and polarisations grids its untuned bits after either was tuned."""
+    from yandasoft_b200 import gridder as G
+    npol = 4
+    ds = _data(npol, 330)
+    acc = G.Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    axes = G.Axes(CELL, CELL)
+    G.autotune_reset()
+    try:
+        fresh = _wproject(6)
+        want = _grid(fresh, npol, lambda g: g.grid(acc))
+        info = fresh.plan(acc).info()
+        more = {"diameter": "12m", "blockage": "1m", "cutoff": 1e-3} if kind == "AWProject" else {}
+        params = {"wmax": 2500.0, "nwplanes": 5, "oversample": os_, "maxsupport": 512, "limitsupport": 6, **more}
+        tuner = make_pair(kind, params if kind != "SphFunc" else {})[1]
+        tuner.initialiseGrid(axes, (NX, NX, npol, 1))
+        rep = tuner.autotune(acc, max_trials=12)
+        assert (rep["cf_width"], rep["npol"]) == (16, npol)
+        g = _wproject(6)
+        assert np.array_equal(_grid(g, npol, lambda g: g.grid(acc)), want)
+        assert g.plan(acc).info() == info
+    finally:
+        G.autotune_reset()

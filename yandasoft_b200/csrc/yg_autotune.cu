@@ -1,9 +1,9 @@
-// Autotuner: picks the uv tile side, the samples per work item and the k_grid
-// thread layout for a CF width class (padded width Wp, polarisations) by
-// timing a degrid + grid pass over a caller's device-resident chunk for each
-// candidate, and remembers the winner for every later gridder of the process
-// with the same class.  No counterpart in the reference (its gridding loop has
-// no such parameters).
+// Autotuner: picks the uv tile side, the samples per work item and the record
+// order and thread layout of the grid kernels for a class of gridders
+// (TuneClass) by timing a degrid + grid pass over a caller's device-resident
+// chunk for each candidate, and remembers the winner for every later gridder
+// of the process of the same class.  No counterpart in the reference (its
+// gridding loop has no such parameters).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,7 +19,7 @@ namespace yg {
 namespace {
 
 std::mutex g_tune_mutex;
-std::map<std::pair<int, int>, TuneChoice> g_tune_table;
+std::map<TuneClass, TuneChoice> g_tune_table;
 
 void throw_if(bool cond, int code, const char* msg) {
   if (cond) throw YgError{code, msg};
@@ -31,17 +31,17 @@ void ck(cudaError_t e, const char* what) {
 
 }  // namespace
 
-bool tune_lookup(int wpad, int npol, TuneChoice* out) {
+bool tune_lookup(const TuneClass& k, TuneChoice* out) {
   std::lock_guard<std::mutex> lk(g_tune_mutex);
-  auto it = g_tune_table.find({wpad, npol});
+  auto it = g_tune_table.find(k);
   if (it == g_tune_table.end()) return false;
   *out = it->second;
   return true;
 }
 
-void tune_store(int wpad, int npol, const TuneChoice& c) {
+void tune_store(const TuneClass& k, const TuneChoice& c) {
   std::lock_guard<std::mutex> lk(g_tune_mutex);
-  g_tune_table[{wpad, npol}] = c;
+  g_tune_table[k] = c;
 }
 
 void tune_clear() {
@@ -58,7 +58,7 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   throw_if(!grids_.p || nx_ == 0, YG_ERR_STATE, "initialiseGrid or initialiseDegrid must come first");
   prepare_plan_cf(dc);
   const int smax = (cf_.maxsize - 1) / 2;
-  const int wpad = ((2 * smax + 1) + 15) / 16 * 16;
+  const TuneClass key = tune_class();
   const int def_tile = grid_tile_for(smax, npol_, cf_.view().varsup != 0);
   std::vector<int> tiles;
   for (int t : {def_tile, def_tile / 2, def_tile * 3 / 4, def_tile * 3 / 2, def_tile * 2}) {
@@ -85,7 +85,7 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   scratch_chunk.vis = model.as<float2>();
   const float* mfs = mfs_weights(dc);
   TuneReport rep;
-  rep.wpad = wpad;
+  rep.wpad = key.wpad;
   rep.npol = npol_;
   cudaEvent_t e0, e1;
   ck(cudaEventCreate(&e0), "event");
@@ -144,7 +144,7 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   vmax_ = save_vmax;
   grid_mode_ = save_mode;
   throw_if(rep.best_ms < 0.f, YG_ERR_UNSUPPORTED, "no candidate ran");
-  tune_store(wpad, npol_, rep.best);
+  tune_store(key, rep.best);
   apply_tuning(rep.best);
   return rep;
 }

@@ -764,13 +764,17 @@ void Gridder::init_cf(const Chunk& dc) {
 // ---------------------------------------------------------------------------
 // binning
 // ---------------------------------------------------------------------------
-// the k_grid thread layout: the caller's, else the autotuner's for this CF
-// width class, else the default
+TuneClass Gridder::tune_class() const {
+  const int smax = (cf_.maxsize - 1) / 2;
+  return TuneClass{((2 * smax + 1) + 15) / 16 * 16, npol_, os_, kind_, kind_ != Kind::AWProject || aw_taper_};
+}
+
+// the record order and thread layout: the caller's, else the autotuner's for
+// this class of gridders, else the default
 int Gridder::grid_variant() const {
   if (grid_mode_ > 0) return grid_mode_;
   TuneChoice c;
-  const int smax = (cf_.maxsize - 1) / 2;
-  if (tune_lookup(((2 * smax + 1) + 15) / 16 * 16, npol_, &c)) return c.variant;
+  if (tune_lookup(tune_class(), &c)) return c.variant;
   return 0;
 }
 
@@ -802,7 +806,7 @@ int Gridder::grid_layout() const {
 int Gridder::tile_for(int smax, int npol) const {
   if (tile_override_ > 0) return tile_override_;
   TuneChoice c;
-  if (tune_lookup(((2 * smax + 1) + 15) / 16 * 16, npol, &c) && c.tile > 0) return c.tile;
+  if (tune_lookup(tune_class(), &c) && c.tile > 0) return c.tile;
   return grid_tile_for(smax, npol, cf_.view().varsup != 0);
 }
 
@@ -916,8 +920,7 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;
-  const int smax_b = (cf_.maxsize - 1) / 2;
-  const bool tuned = tune_lookup(((2 * smax_b + 1) + 15) / 16 * 16, npol_, &tc);
+  const bool tuned = tune_lookup(tune_class(), &tc);
   if (vmax <= 0 && tuned && tile_override_ <= 0) vmax = tc.vmax;
   if (vmax <= 0) {
     const long long n = dc.nrow * (long long)dc.nchan;

@@ -6,6 +6,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "yg_cf.h"
@@ -85,8 +86,20 @@ struct TuneReport {
   float best_ms = -1.f, default_ms = -1.f;
   std::vector<TuneTrial> trials;
 };
-bool tune_lookup(int wpad, int npol, TuneChoice* out);
-void tune_store(int wpad, int npol, const TuneChoice& c);
+// What a choice holds for: the padded CF width and polarisations set the tile
+// and the thread layouts; the gridder kind, its oversampling and whether its
+// images are corrected set which kernels take its CF table, which of them is
+// the faster and whether a change of the record order may be seen in an image.
+struct TuneClass {
+  int wpad, npol, os;
+  Kind kind;
+  bool corrected;
+  bool operator<(const TuneClass& o) const {
+    return std::tie(wpad, npol, os, kind, corrected) < std::tie(o.wpad, o.npol, o.os, o.kind, o.corrected);
+  }
+};
+bool tune_lookup(const TuneClass& k, TuneChoice* out);
+void tune_store(const TuneClass& k, const TuneChoice& c);
 void tune_clear();
 
 class Gridder {
@@ -154,6 +167,7 @@ class Gridder {
   void set_tile(int t) { tile_override_ = t; }
   void set_grid_mode(int m) { grid_mode_ = m; }
   int tile_for(int smax, int npol) const;
+  TuneClass tune_class() const;
   int grid_variant() const;
   int grid_layout() const;
   int items_vmax() const { return vmax_; }
