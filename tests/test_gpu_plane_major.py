@@ -146,3 +146,25 @@ def test_cf_major_same_sums(support, os_, npol, tile, item, diameter, mode):
     _adopt_cf(og, gg)
     og.grid(chunk)
     assert rel_l2(out[0], np.stack(og.grids)) < TOL
+
+
+@pytest.mark.parametrize("support,os_,npol,tile", [(37, 4, 1, 56), (23, 4, 1, 108), (22, 4, 1, 28)])
+def test_cf_major_full_ring(support, os_, npol, tile):
+    """Widths and tiles at which k_grid_cf's ring fills its shared-memory
+    budget to the byte, the kernel's static shared memory included."""
+    from yandasoft_b200.gridder import Accessor, Axes
+    ds, flag, noise, delay = _inputs(npol, 600.0, 200 + support)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis, noise=noise, flag=flag, delay=delay).to_device()
+    out = []
+    params = {"wmax": 9000.0, "nwplanes": 5, "oversample": os_, "maxsupport": 1024, "limitsupport": support}
+    for variant in (0, 64):
+        _, gg = make_pair("WProject", params)
+        gg.set_tile(tile)
+        gg.set_grid_variant(variant)
+        gg.initialiseGrid(Axes(CELL, CELL), (NX, NX, npol, 1))
+        gg.grid(acc)
+        assert gg.support()[0] == support
+        out.append((np.stack(gg.grids()), gg.sum_weights()))
+    assert np.abs(out[1][0]).max() > 0
+    assert rel_l2(out[0][0], out[1][0]) < TOL
+    assert np.array_equal(out[0][1], out[1][1])

@@ -1075,12 +1075,15 @@ CfShape cf_shape(int W, int P, int npol, bool few) {
       s.cfs = cfs;
       s.stage = cf_stage_bytes(cfs ? cf_b : 0, npa);
       const size_t slot = (((size_t)P * P * npa + 1) & ~(size_t)1) * sizeof(float2);
-      const size_t fixed = slot + 448 + fetch_bytes(npa);   // (with the static shared memory)
+      const size_t fixed = slot + 448 + fetch_bytes(npa);   // (with roundings and the kernel's static shared memory)
       const int want = cfs && cf_b > 8192 ? 2 : 4;
       if (fixed + want * (size_t)(s.stage + 16) > budget) continue;
       if (!cf_threads((cfs ? (W + 7) / 8 * 8 : W) * W, npa, ctas, &s)) continue;
       s.nstages = (int)std::min<size_t>(8, (budget - fixed) / (s.stage + 16));
-      s.smem = fixed + s.nstages * (size_t)(s.stage + 16);
+      // what the kernel addresses: its static shared memory comes on top of the
+      // dynamic size, which must leave it its part of the budget (a ring that
+      // fills the budget to the byte would not launch: W 75, tile 56)
+      s.smem = (slot + 127) / 128 * 128 + s.nstages * (size_t)(s.stage + 16) + fetch_bytes(npa);
       return s;
     }
   }
