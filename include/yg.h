@@ -176,7 +176,7 @@ int yg_set_item_size(yg_gridder* g, int32_t vmax); /* samples per work item */
  * (plans made afterwards keep both orders) and reads the taps through L2;
  * 64 (the other bits up to 128 are then ignored) orders them by CF plane, then
  * position, then oversampling offset and keeps each footprint's running sums in
- * registers (k_grid_pl; CFs of one common size).
+ * registers (k_grid_pl; CFs of one common size, others are gridded as with 1).
  * Adding 256 degrids 16-wide CFs with the CF read per tap from the segment
  * ring (k_degrid_t) instead of the default register-held CF column; adding
  * 512 has the default degrid one sample per half-warp pass instead of two. */

@@ -80,3 +80,24 @@ def test_tuning_serves_its_own_class(kind, os_):
         assert g.plan(acc).info() == info
     finally:
         G.autotune_reset()
+
+
+@pytest.mark.parametrize("npol", [1, 4])
+@pytest.mark.parametrize("variant", [64, 65, 66, 67, 80, 194])
+def test_plane_major_bits_beside(npol, variant):
+    """Bit 64 stands alone: the bits up to 128 beside it change nothing, and a
+    table that the plane-major kernel does not take (CFs of several sizes, up
+    to 16 wide) is gridded as with variant 1, bit for bit."""
+    from yandasoft_b200.gridder import Accessor
+    ds = _data(npol, 340)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    for more, same in (({}, 64), ({"variablesupport": True}, 1)):
+        out = []
+        for v in (variant, same):
+            g = _wproject(6, **more)
+            g.set_grid_variant(v)
+            out.append(_grid(g, npol, lambda g: g.grid(acc)))
+        sizes = {c.shape for c in g.convolution_functions() if c is not None}
+        assert (len(sizes) > 1) == bool(more)
+        assert np.abs(out[1]).max() > 0
+        assert np.array_equal(out[0], out[1])

@@ -360,9 +360,9 @@ int yg_set_grid_variant(yg_gridder* g, int32_t variant) {
   return guarded([&] {
     if (variant < 0 || (variant & ~(240 | 256 | 512)) > 3)
       throw yg::YgError{YG_ERR_ARG, "variant must be 0 to 3, plus 16 (register accumulation), 32 "
-                                    "(position-major records) or 64 (plane-major records, staged CF planes; "
-                                    "plus 128: their tile in global memory), plus 256 (degridding by "
-                                    "k_degrid_t) or 512 (one degridded sample per half-warp pass)"};
+                                    "(position-major records) or 64 (plane-major records; the bits up to 128 "
+                                    "beside it are ignored), plus 256 (degridding by k_degrid_t) or 512 (one "
+                                    "degridded sample per half-warp pass)"};
     G(g).set_grid_mode(variant);
   });
 }

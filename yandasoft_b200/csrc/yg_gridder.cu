@@ -787,20 +787,30 @@ int Gridder::cf_mode() const {
   }
 }
 
-// grid_variant() with the automatic choice made: plane-major records (64) for
-// AWProject where the plane-major kernel takes the CF table, CF-major (1)
-// otherwise.  The other gridders' images are divided by the spheroidal, whose
-// factors of 10^4 in the corners turn the rounding of another order of a
-// cell's sum into 1e-4 of the image: their automatic choice keeps the CF-major
-// order, so that an image stays what it was bit for bit, and the plane-major
-// order is theirs to ask for or tune to.  Plans are made by this choice and
-// passes run by it: the records that a plan happens to hold decide nothing.
+// Whether the plane-major kernel serves this gridder's CFs.
+bool Gridder::takes_planes() const {
+  return cf_form_ == 0 && grid_pl_block(cf_.view(), os_, cf_mode(), npol_) != 0;
+}
+
+// The automatic choice: plane-major records (64) for AWProject where the
+// plane-major kernel takes the CF table, CF-major (1) otherwise.  The other
+// gridders' images are divided by the spheroidal, whose factors of 10^4 in the
+// corners turn the rounding of another order of a cell's sum into 1e-4 of the
+// image: their automatic choice keeps the CF-major order, so that an image
+// stays what it was bit for bit, and the plane-major order is theirs to ask for
+// or tune to.
+int Gridder::automatic_layout() const {
+  return kind_ == Kind::AWProject && !aw_taper_ && takes_planes() ? 64 : 1;
+}
+
+// grid_variant() as plans are made by it and passes run by it (the records that
+// a plan happens to hold decide nothing): the automatic choice made, and with
+// bit 64 no other bit up to 128, or the CF-major layout where the plane-major
+// kernel does not take the CF table.
 int Gridder::grid_layout() const {
-  const int v = grid_variant();
-  if ((v & 255) != 0) return v;
-  const bool planes = kind_ == Kind::AWProject && !aw_taper_ && cf_form_ == 0 &&
-                      grid_pl_block(cf_.view(), os_, cf_mode(), npol_) != 0;
-  return v | (planes ? 64 : 1);
+  const int v = grid_variant(), degrid = v & ~255;
+  if ((v & 255) == 0) return degrid | automatic_layout();
+  return v & 64 ? degrid | (takes_planes() ? 64 : 1) : v;
 }
 
 int Gridder::tile_for(int smax, int npol) const {
@@ -842,10 +852,9 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   // unless a layout of several slots per thread was asked for
   const int wpad16 = ((2 * smax + 1) + 15) / 16 * 16;
   const int variant = grid_layout();
-  a.wy = (wpad16 == 16 && ((variant & 15) <= 1 || (variant & 64)) && exact_rows_) ? 2 * smax + 1 : 0;
-  // records for the plane-major kernel where it takes the table
-  a.pl_fs = (variant & 64) && cf_form_ == 0 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
-  a.pos_major = a.pl_fs != 0 ? 2 : ((variant & 32) && !(variant & 64) ? 1 : 0);
+  a.wy = (wpad16 == 16 && (variant & 15) <= 1 && exact_rows_) ? 2 * smax + 1 : 0;
+  a.pl_fs = variant & 64 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
+  a.pos_major = variant & 64 ? 2 : (variant & 32 ? 1 : 0);
   a.key_planes = 0;
   a.keep_inv = 1;
   a.ntx = (nx_ + a.tile - 1) / a.tile;

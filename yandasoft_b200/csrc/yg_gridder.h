@@ -205,6 +205,8 @@ class Gridder {
   std::vector<int> chan_map(const double* freq_host, int nchan) const;
   void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
   int cf_mode() const;
+  bool takes_planes() const;
+  int automatic_layout() const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
   int corr_nx_ = 0, corr_ny_ = 0;      // shape that corr_d_ was made for
