@@ -101,3 +101,26 @@ def test_plane_major_bits_beside(npol, variant):
         assert (len(sizes) > 1) == bool(more)
         assert np.abs(out[1]).max() > 0
         assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("kind,support", [("AWProject", 6), ("WProject", 6)])
+def test_tuner_times_the_automatic_choice(kind, support):
+    """default_ms is the time of what an untuned handle runs (plane-major for
+    AWProject, CF-major for the others): with one trial it is that trial's, and
+    the choice kept grids the untuned bits."""
+    from yandasoft_b200 import gridder as G
+    ds = _data(2, 350)
+    acc = G.Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    more = {"diameter": "12m", "blockage": "1m", "cutoff": 1e-3} if kind == "AWProject" else {}
+    params = {"wmax": 2500.0, "nwplanes": 5, "oversample": 4, "maxsupport": 512, "limitsupport": support, **more}
+    G.autotune_reset()
+    try:
+        want = _grid(make_pair(kind, params)[1], 2, lambda g: g.grid(acc))
+        tuner = make_pair(kind, params)[1]
+        tuner.initialiseGrid(G.Axes(CELL, CELL), (NX, NX, 2, 1))
+        rep = tuner.autotune(acc, max_trials=1)
+        assert rep["trials"] == 1 and rep["variant"] == (64 if kind == "AWProject" else 1)
+        assert rep["default_ms"] == rep["best_ms"] > 0
+        assert np.array_equal(_grid(tuner, 2, lambda g: g.grid(acc)), want)
+    finally:
+        G.autotune_reset()

@@ -76,7 +76,10 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   // registers (17).  Position-major records with taps
   // through L2 (32) measured slower on the benchmark workloads and are not
   // tried.
-  const std::vector<int> variants{1, 64, 17, 2};
+  std::vector<int> variants{1, 64, 17, 2};
+  // the automatic choice comes first: the trial that default_ms reports
+  const int def_variant = automatic_layout();
+  std::stable_partition(variants.begin(), variants.end(), [&](int v) { return v == def_variant; });
   const int save_tile = tile_override_, save_vmax = vmax_, save_mode = grid_mode_;
   Chunk scratch_chunk = dc;
   DevBuf model;
@@ -126,7 +129,7 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
       rep.best_ms = ms;
       rep.best = TuneChoice{t, vm, v};
     }
-    if (t == def_tile && vm == def_vmax && v == 1) rep.default_ms = ms;
+    if (t == def_tile && vm == def_vmax && v == def_variant) rep.default_ms = ms;
   };
   // the layouts at the default tile (the default first), then the other tiles
   // with the best layout, then the work-item size around the best of those
