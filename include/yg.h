@@ -149,7 +149,9 @@ int64_t yg_kernel_launch_count(void);
  * (SphFunc, WProject, WStack; AWProject builds from data). */
 int yg_build_cf(yg_gridder* g);
 
-/* ---- plans: bin a chunk once, grid/degrid it many times (major cycle) ---- */
+/* ---- plans: bin a chunk once, grid/degrid it many times (major cycle) ----
+ * A plan serves one pass at a time: passes over it by several handles follow
+ * one another, from one thread or under the caller's lock. */
 int yg_plan_create(yg_gridder* g, const yg_chunk* chunk, yg_plan** out);
 int yg_plan_grid(yg_gridder* g, const yg_plan* plan, const yg_chunk* chunk);
 int yg_plan_degrid(yg_gridder* g, yg_plan* plan, yg_chunk* chunk);

@@ -124,3 +124,45 @@ def test_tuner_times_the_automatic_choice(kind, support):
         assert np.array_equal(_grid(tuner, 2, lambda g: g.grid(acc)), want)
     finally:
         G.autotune_reset()
+
+
+@pytest.mark.parametrize("more,variant", [({"variablesupport": True}, 0), ({}, 2), ({}, 17)])
+def test_inverse_is_made_with_the_plan(more, variant):
+    """Layouts and tables whose kernel reads the inverse permutation get it with
+    the plan, before any pass: the first pass over a plan launches what every
+    later one does."""
+    from yandasoft_b200 import gridder as G
+    ds = _data(2, 360)
+    acc = G.Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    g = _wproject(6, **more)
+    g.set_grid_variant(variant)
+    g.initialiseGrid(G.Axes(CELL, CELL), (NX, NX, 2, 1))
+    plan = g.plan(acc)
+    n, out = [], []
+    for _ in range(2):
+        before = G.kernel_launch_count()
+        out.append(_grid(g, 2, lambda g: g.grid_plan(plan, acc)))
+        n.append(G.kernel_launch_count() - before)
+    assert n[0] == n[1]
+    assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
+
+
+def test_inverse_for_another_layout():
+    """A plan made under the automatic choice has no inverse permutation; the
+    first pass that needs it makes it, and the next one, of another handle on
+    another stream, finds it complete."""
+    from yandasoft_b200.gridder import Accessor, Axes
+    ds = _data(4, 370)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    a, b = _wproject(6), _wproject(6)
+    a.initialiseGrid(Axes(CELL, CELL), (NX, NX, 4, 1))
+    want = _grid(a, 4, lambda g: g.grid(acc))
+    for variant in (16, 17):
+        ref = _wproject(6)
+        ref.set_grid_variant(variant)
+        want = _grid(ref, 4, lambda g: g.grid(acc))
+        plan = a.plan(acc)
+        for g in (a, b, a):
+            g.set_grid_variant(variant)
+            assert np.array_equal(_grid(g, 4, lambda g: g.grid_plan(plan, acc)), want)
+        a.set_grid_variant(0)

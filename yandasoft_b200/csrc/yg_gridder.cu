@@ -926,6 +926,13 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // a gridding-only plan for the plane-major kernel sorts once, by its key
   a.key_planes = (use == PLAN_GRID && a.pos_major == 2) ? 1 : 0;
   a.keep_inv = use != PLAN_DEGRID ? 1 : 0;
+  // k_grid runs the layouts that are asked for, the learned CF and the tables
+  // that neither of the other kernels takes (the position-major layout has an
+  // inverse of its own)
+  const int layout = grid_layout() & 255;
+  a.need_inv = a.keep_inv && (cf_form_ != 0 || (layout != 64 && !(layout & 32) &&
+                                                (layout != 1 || !grid_cf_takes(a.cf, a.tile + a.cf.maxsize - 1,
+                                                                               npol_, os_))));
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;

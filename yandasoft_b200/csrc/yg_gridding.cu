@@ -1785,6 +1785,39 @@ __global__ void k_plan_counts(const int* __restrict__ last_base, const int* __re
   out[1] = *nvalid;
 }
 
+// The inverse permutation of the CF-major records (sample id -> sorted slot),
+// which k_grid's gather reads; k_grid_cf and k_grid_pl need none.
+static int enqueue_inverse(Plan& pl, cudaStream_t st) {
+  YG_CUDA_TRY(pl.inv.ensure((size_t)pl.nsamples * 4));
+  YG_CUDA_TRY(cudaMemsetAsync(pl.inv.p, 0xff, (size_t)pl.nsamples * 4, st));
+  if (pl.nvalid > 0) {
+    k_inverse<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(pl.rec.as<int4>(), pl.nvalid, pl.inv.as<int>());
+    YG_COUNT_LAUNCH();
+    YG_CUDA_TRY(cudaGetLastError());
+  }
+  return YG_OK;
+}
+
+// A pass in another layout than its plan was made for (a plan made under the
+// automatic choice, gridded under variant 2): the first one builds the inverse
+// and waits for it before anyone may see it as ready, since the next may come
+// from another handle, on another stream.  A stream capture cannot wait; the
+// uncaptured pass before it has built the inverse.
+static int inverse_for_pass(const Plan& plan, cudaStream_t st) {
+  Plan& pl = const_cast<Plan&>(plan);
+  std::lock_guard<std::mutex> lk(pl.inv_mutex);
+  if (pl.inv_ready) return YG_OK;
+  if (!pl.keep_inv) return YG_ERR_STATE;   // a plan made for degridding only
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  YG_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return YG_ERR_STATE;
+  const int rc = enqueue_inverse(pl, st);
+  if (rc) return rc;
+  YG_CUDA_TRY(cudaStreamSynchronize(st));
+  pl.inv_ready = true;
+  return YG_OK;
+}
+
 // Bins one chunk: fills plan (sorted ids, tile table, work items).
 int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t st) {
   const long long n = a.nrow * (long long)a.nchan;
@@ -1884,6 +1917,12 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
   }
   pl.inv_ready = pl.inv_pos_ready = false;
   pl.keep_inv = a.keep_inv != 0;
+  if (a.need_inv) {
+    // the caller waits for the plan before any pass reads it
+    const int rc = enqueue_inverse(pl, st);
+    if (rc) return rc;
+    pl.inv_ready = true;
+  }
   pl.pos_ready = false;
   pl.grid_only = false;
   if (a.key_planes) {
@@ -2228,18 +2267,10 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
   if (v.npol > 4) return YG_ERR_UNSUPPORTED;
   // the weighted visibilities in the order of the records the kernel reads,
   // gathered in the cube's order; the weight checks and the sums of weights
-  // over the sorted records.  The inverse permutation is built when a pass
-  // first asks for it (k_grid_cf and k_grid_pl need none).
-  if (!pos && !pl.inv_ready) {
-    Plan& p = const_cast<Plan&>(pl);
-    if (!p.keep_inv) return YG_ERR_STATE;   // a plan made for degridding only
-    YG_CUDA_TRY(p.inv.ensure((size_t)pl.nsamples * 4));
-    YG_CUDA_TRY(cudaMemsetAsync(p.inv.p, 0xff, (size_t)pl.nsamples * 4, st));
-    if (pl.nvalid > 0) {
-      k_inverse<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(pl.rec.as<int4>(), pl.nvalid, p.inv.as<int>());
-      YG_COUNT_LAUNCH();
-    }
-    p.inv_ready = true;
+  // over the sorted records
+  if (!pos) {
+    const int rc = inverse_for_pass(pl, st);
+    if (rc) return rc;
   }
   YG_CUDA_TRY(svis.ensure_headroom((size_t)std::max(1ll, pl.nvalid) * v.npol * sizeof(float2)));
   k_gather_cube<<<grid_dim(pl.nsamples, 256), 256, 0, st>>>(v, pos ? pl.inv_pos.as<int>() : pl.inv.as<int>(),

@@ -1,6 +1,7 @@
 // Internal (non-ABI) structures of the B200 gridder shared by the host
 // classes and the CUDA kernels.
 #pragma once
+#include <mutex>
 #include <cstddef>
 #include <cstdint>
 #include <string>
@@ -122,6 +123,7 @@ struct BinArgs {
   int pl_fs;               // plane-major order: matrices per CF plane (grid_pl_block)
   int key_planes;          // a plan for gridding only: sort once, by the plane-major key (pos_major 2)
   int keep_inv;            // the CF-major records may be gridded: their inverse permutation can be built later
+  int need_inv;            // it is built with the plan: the layout and the CF table are k_grid's
   unsigned long long invalid_key;  // one past the largest valid key
   CFView cf;
 };
@@ -154,6 +156,7 @@ struct Plan {
   bool grid_only = false;       // sorted once, plane-major: rec_pos only (no CF-major records)
   bool inv_ready = false, inv_pos_ready = false;   // inv / inv_pos are built
   bool keep_inv = false;        // inv may be built when a pass first needs it
+  std::mutex inv_mutex;         // held by the pass that builds it
   int pos_mode = 0;             // its order: 1 position then CF index; 2 CF plane, position, offset
   int pl_fs = 0;                // plane-major records: grid_pl_block of their CF table
   DevBuf ext;                   // continuous learned CF: per sorted sample (ru, rv, w, 0)
