@@ -130,3 +130,27 @@ def test_model_empty(on_device, where):
     assert g.isModelEmpty() == (where is None)
     if where is None:
         assert not np.any(g.grids()[0])
+
+
+def test_corrections_follow_the_shape():
+    """One handle through several shapes, host and device models in turn: the
+    first pass after each change takes the new shape's correction factors (the
+    grids and images of a handle that never had another shape)."""
+    import torch
+    G, g, axes = setup("SphFunc", 64, 64, 1, 1, 1.0)
+    rng = np.random.default_rng(7)
+    uvw = rng.uniform(-400, 400, (200, 3))
+    vis = np.asfortranarray(rng.standard_normal((200, 1, 1)), dtype=np.complex64)
+    acc = G.Accessor(uvw, np.array([1.0e9]), vis)
+    for k, (nx, ny) in enumerate([(90, 66), (128, 64), (66, 90), (256, 256), (64, 128), (90, 66)]):
+        img = np.asfortranarray(rng.standard_normal((nx, ny, 1, 1)), dtype=np.float32)
+        give = torch.from_numpy(np.ascontiguousarray(img.transpose(3, 2, 1, 0))).cuda().permute(3, 2, 1, 0) \
+            if k % 2 else img
+        fresh = setup("SphFunc", nx, ny, 1, 1, 1.0)[1]
+        for h in (g, fresh):
+            h.initialiseDegrid(axes, give)
+        assert np.array_equal(g.grids()[0], fresh.grids()[0])
+        for h in (g, fresh):
+            h.initialiseGrid(axes, (nx, ny, 1, 1))
+            h.grid(acc)
+        assert np.array_equal(g.finaliseGrid(), fresh.finaliseGrid())

@@ -1268,8 +1268,15 @@ void Gridder::prepare_corrections() {
   const std::vector<double> cx = sph_correction(nx_, g), cy = nx_ == ny_ ? cx : sph_correction(ny_, g);
   corr_nx_ = corr_ny_ = 0;
   cuda_check(corr_d_.ensure((nx_ + ny_) * sizeof(double)), "alloc");
-  cuda_check(cudaMemcpy(corr_d_.p, cx.data(), nx_ * sizeof(double), cudaMemcpyHostToDevice), "up");
-  cuda_check(cudaMemcpy(corr_d_.as<double>() + nx_, cy.data(), ny_ * sizeof(double), cudaMemcpyHostToDevice), "up");
+  // on the handle's stream, where the passes that read them run: a copy on
+  // another stream may return before the factors have arrived (pageable source,
+  // staged by the call) and nothing would order it before those passes, or
+  // after the ones still reading the factors of the shape before
+  auto up = [&](double* dst, const std::vector<double>& v) {
+    cuda_check(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice, stream_), "up");
+  };
+  up(corr_d_.as<double>(), cx);
+  up(corr_d_.as<double>() + nx_, cy);
   corr_nx_ = nx_;
   corr_ny_ = ny_;
 }
