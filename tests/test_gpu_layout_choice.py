@@ -166,3 +166,23 @@ def test_inverse_for_another_layout():
             g.set_grid_variant(variant)
             assert np.array_equal(_grid(g, 4, lambda g: g.grid_plan(plan, acc)), want)
         a.set_grid_variant(0)
+
+
+@pytest.mark.parametrize("kind,variant", [("AWProject", 0), ("WProject", 64)])
+def test_slot_beyond_32_bits(kind, variant):
+    """A tile whose slot the plane-major kernel cannot index (4 polarisations,
+    (23200 + 12)^2 cells: above 2^31 elements) is refused, as by variant 1."""
+    from yandasoft_b200 import gridder as G
+    ds = _data(4, 380)
+    acc = G.Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    more = {"diameter": "12m", "blockage": "1m", "cutoff": 1e-3} if kind == "AWProject" else {}
+    params = {"wmax": 2500.0, "nwplanes": 5, "oversample": 4, "maxsupport": 512, "limitsupport": 6, **more}
+    for v in (variant, 1):
+        g = make_pair(kind, params)[1]
+        g.set_tile(23200)
+        g.set_item_size(1 << 20)
+        g.set_grid_variant(v)
+        g.initialiseGrid(G.Axes(CELL, CELL), (NX, NX, 4, 1))
+        with pytest.raises(G.AskapError) as e:
+            g.grid(acc)
+        assert e.value.code == 9

@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(NPOL == 1 ? 416 : (SL <= 4 ? 288 : 256), NPOL 
   if (warp == ntap) {
     // ---- producer
     const unsigned fm = 0xffffffffu;
-    // coordinates below 2^12 divide exactly by W through this reciprocal: the
-    // product is at least k for x = k W and below k + 1 for x = k W + W - 1
+    // coordinates below 2^16 (a record holds no more) divide exactly by W
+    // through this reciprocal: the product is at least k for x = k W and below
+    // k + 1 for x = k W + W - 1 (every x and W checked, W up to 1032)
     const float rW = __frcp_rn((float)W) * (1.f + 1e-6f);
     int seg = 0, cur = -1, nblock = 0, why = 1;
     bool ok = true;

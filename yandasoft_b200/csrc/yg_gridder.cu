@@ -787,9 +787,13 @@ int Gridder::cf_mode() const {
   }
 }
 
-// Whether the plane-major kernel serves this gridder's CFs.
+// Whether the plane-major kernel serves this gridder's CFs: no learned form, a
+// table that it takes, and a slot (tile and halo, all polarisations) whose
+// elements it can index with 32 bits, whatever tile was asked for.
 bool Gridder::takes_planes() const {
-  return cf_form_ == 0 && grid_pl_block(cf_.view(), os_, cf_mode(), npol_) != 0;
+  const CFView cf = cf_.view();
+  const long long pad = tile_for((cf.maxsize - 1) / 2, npol_) + cf.maxsize - 1ll;
+  return cf_form_ == 0 && pad * pad * npol_ <= 0x7fffffffll && grid_pl_block(cf, os_, cf_mode(), npol_) != 0;
 }
 
 // The automatic choice: plane-major records (64) for AWProject where the
