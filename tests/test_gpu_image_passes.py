@@ -154,3 +154,34 @@ def test_corrections_follow_the_shape():
             h.initialiseGrid(axes, (nx, ny, 1, 1))
             h.grid(acc)
         assert np.array_equal(g.finaliseGrid(), fresh.finaliseGrid())
+
+
+@pytest.mark.parametrize("on_device", [False, True])
+def test_empty_model_is_not_transformed(on_device):
+    """An empty model costs a look at it and cleared grids, not the screens and
+    transforms of its 17 grids: less than half of what another model takes (the
+    transforms alone are several times the rest)."""
+    import time
+    import torch
+    from yandasoft_b200 import gridder as G
+    n = 2048
+    g = G.VisGridderFactory.make({"gridder": "WStack", "gridder.WStack.wmax": 2000.0, "gridder.WStack.nwplanes": 17})
+    axes = G.Axes(CELL, CELL)
+    best = {}
+    for value in (1.0, 0.0):
+        img = np.zeros((n, n, 1, 1), dtype=np.float32, order="F")
+        img[n // 2 + 3, n // 2 - 7, 0, 0] = value
+        give = torch.from_numpy(np.ascontiguousarray(img.transpose(3, 2, 1, 0))).cuda().permute(3, 2, 1, 0) \
+            if on_device else torch.from_numpy(np.ascontiguousarray(img.transpose(3, 2, 1, 0))).pin_memory().numpy() \
+            .transpose(3, 2, 1, 0)
+        times = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            g.initialiseDegrid(axes, give)
+            times.append(time.perf_counter() - t0)
+        assert g.isModelEmpty() == (value == 0.0)
+        best[value] = min(times[1:])
+    print("initialiseDegrid %s: %.3f ms, empty %.3f ms" % (on_device, 1e3 * best[1.0], 1e3 * best[0.0]))
+    upload = 0.0 if on_device else 1e-3 * n * n * 4 / 40e6      # 17 MB at 40 GB/s and above
+    assert best[0.0] - upload < 0.5 * (best[1.0] - upload)

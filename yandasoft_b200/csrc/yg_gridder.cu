@@ -413,6 +413,7 @@ Gridder::~Gridder() {
     if (e) cudaEventDestroy(e);
   if (piece_binned_) cudaEventDestroy(piece_binned_);
   if (legacy_ev_) cudaEventDestroy(legacy_ev_);
+  if (any_ev_) cudaEventDestroy(any_ev_);
   if (stream_) {
     cudaStreamSynchronize(stream_);
     cudaStreamDestroy(stream_);
@@ -1398,10 +1399,12 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   const long long total = (long long)nx_ * ny_ * nplanes;
   const size_t gbytes = (size_t)ngrids() * total * sizeof(float2);
   cuda_check(grids_.ensure(gbytes), "alloc grids");
-  // the model image on the device: the caller's, or an upload of it; the
-  // first pass over it also tells whether it is empty
+  // the model image on the device: the caller's, or an upload of it; the first
+  // pass over it also tells whether it is empty
   cuda_check(img_tmp_.ensure(64 + (on_device ? 0 : in_total * sizeof(float))), "alloc");
-  int* any = img_tmp_.as<int>();
+  cuda_check(any_h_.ensure(sizeof(int)), "alloc");
+  if (!any_ev_) cuda_check(cudaEventCreateWithFlags(&any_ev_, cudaEventDisableTiming), "event");
+  const ModelFlag flag{img_tmp_.as<int>(), any_h_.as<volatile int>(), any_ev_};
   const float* dimg = image;
   if (on_device) {
     order_after_legacy_stream();
@@ -1410,7 +1413,7 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
     cuda_check(cudaMemcpyAsync(up, image, in_total * sizeof(float), cudaMemcpyHostToDevice, stream_), "upload model");
     dimg = up;
   }
-  cuda_check(cudaMemsetAsync(any, 0, sizeof(int), stream_), "memset");
+  cuda_check(cudaMemsetAsync(flag.dev, 0, sizeof(int), stream_), "memset");
   prepare_corrections();
   std::vector<StackScreen> screens;
   const std::vector<StackScreen>* sp = nullptr;
@@ -1421,19 +1424,14 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   }
   const double* cx = corr_d_.p ? corr_d_.as<double>() : nullptr;
   const double* cy = corr_d_.p ? corr_d_.as<double>() + nx_ : nullptr;
-  rc_check(image_to_grids(fft_, dimg, nx, ny, nx_, ny_, nplanes, sp, ngrids(), cx, cy, grids_.as<float2>(), any,
+  rc_check(image_to_grids(fft_, dimg, nx, ny, nx_, ny_, nplanes, sp, ngrids(), cx, cy, grids_.as<float2>(), flag,
                           stream_),
            "initialiseDegrid");
-  int seen = 0;
-  cuda_check(cudaMemcpyAsync(&seen, any, sizeof(int), cudaMemcpyDeviceToHost, stream_), "model check");
+  model_empty_ = *flag.host == 0;
+  if (model_empty_) cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
   sync();
-  model_empty_ = seen == 0;
-  if (model_empty_) {
-    cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
-    sync();
-    return;
-  }
-  throw_if(nx > nx_ || ny > ny_, YG_ERR_CUDA, "initialiseDegrid: the padded grid is smaller than the image");
+  throw_if(!model_empty_ && (nx > nx_ || ny > ny_), YG_ERR_CUDA,
+           "initialiseDegrid: the padded grid is smaller than the image");
 }
 
 void Gridder::finalise_degrid() {

@@ -279,6 +279,7 @@ class Gridder {
   LearnedCF learned_view_for(const Chunk& dc, Plan& pl);
   DevBuf grids_, sumw_, carry_, err_, chanmap_d_, rowok_d_, corr_d_;
   HostMapped err_h_;                   // mapped host mirror of err_ for the read-back
+  HostMapped any_h_;                   // whether a pixel of the model differs from zero
   std::vector<float> mfs_w_;           // host MFS weights of the last upload
   std::vector<double> mfs_freqs_;      // frequencies they were made for
   int mfs_key_order_ = -1;
@@ -309,6 +310,7 @@ class Gridder {
   ImageFFT fft_;
   cudaStream_t stream_ = nullptr;
   cudaEvent_t legacy_ev_ = nullptr;
+  cudaEvent_t any_ev_ = nullptr;       // any_h_ holds the latest model's answer
   Stats stats_;
   int device_ = 0;
   bool device_ready_ = false;

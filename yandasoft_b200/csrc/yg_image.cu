@@ -233,7 +233,7 @@ int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny,
 
 int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, int ny, int nplanes,
                    const std::vector<StackScreen>* screens, int ngrids, const double* corr_x, const double* corr_y,
-                   float2* grids, int* any, cudaStream_t st) {
+                   float2* grids, const ModelFlag& flag, cudaStream_t st) {
   int rc = f.ensure(nx, ny, nplanes, st);
   if (rc) return rc;
   const long long total = (long long)nx * ny * nplanes;
@@ -244,10 +244,21 @@ int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, in
     const bool use = screens != nullptr;
     k_image_to_uv<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(image, dst, inx, iny, nx, ny, nplanes, roll, use,
                                                              use ? (*screens)[g] : StackScreen{},
-                                                             corr ? corr_x : nullptr, corr_y, g == 0 ? any : nullptr);
+                                                             corr ? corr_x : nullptr, corr_y, g == 0 ? flag.dev : nullptr);
+    if (g == 0) {
+      IM_TRY(cudaMemcpyAsync((void*)flag.host, flag.dev, sizeof(int), cudaMemcpyDeviceToHost, st));
+      IM_TRY(cudaEventRecord(flag.copied, st));
+    }
     if (cufftExecC2C(f.plan, (cufftComplex*)dst, (cufftComplex*)dst, CUFFT_FORWARD) != CUFFT_SUCCESS) return YG_ERR_CUDA;
     if (!roll)
       k_checkerboard<<<dim3((nx + 255) / 256, ny), 256, 0, st>>>(dst, dst, nx, ny, nplanes, nx / 2 + ny / 2);
+    // an empty model (the first cycle of every clean) makes no other grid; the
+    // host learns of it while the first transform runs, so that nothing waits
+    // (17 grids of 4096^2 x 4, empty: 2.0 ms, 13.6 with all of their transforms)
+    if (g == 0) {
+      IM_TRY(cudaEventSynchronize(flag.copied));
+      if (*flag.host == 0) break;
+    }
   }
   IM_TRY(cudaGetLastError());
   return YG_OK;

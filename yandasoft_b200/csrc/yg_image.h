@@ -30,12 +30,20 @@ struct ImageFFT {
 int image_finalise(ImageFFT& f, const float2* grids, int ngrids, int nx, int ny, int nplanes,
                    const std::vector<StackScreen>* screens, const double* corr_x, const double* corr_y, float* out,
                    int onx, int ony, cudaStream_t st);
+// Whether a pixel of the model differs from zero: a flag that the first image
+// pass sets, copied to pinned host memory and waited for by its own event.
+struct ModelFlag {
+  int* dev;
+  volatile int* host;
+  cudaEvent_t copied;
+};
 // grids_g = forward FFT of the device image (inx, iny, nplanes) in the centre
-// of (nx, ny), corrected, times screen_g; *any (device) is set when a pixel is
-// not zero
+// of (nx, ny), corrected, times screen_g; *flag.host tells after the call
+// whether the part of the image inside (nx, ny) is empty, and if it is the
+// grids are not made
 int image_to_grids(ImageFFT& f, const float* image, int inx, int iny, int nx, int ny, int nplanes,
                    const std::vector<StackScreen>* screens, int ngrids, const double* corr_x, const double* corr_y,
-                   float2* grids, int* any, cudaStream_t st);
+                   float2* grids, const ModelFlag& flag, cudaStream_t st);
 
 // every pixel of plane p of out (npix per plane, device) = vals[p]
 int fill_planes(float* out, long long npix, const std::vector<float>& vals, cudaStream_t st);
