@@ -185,3 +185,25 @@ def test_empty_model_is_not_transformed(on_device):
     print("initialiseDegrid %s: %.3f ms, empty %.3f ms" % (on_device, 1e3 * best[1.0], 1e3 * best[0.0]))
     upload = 0.0 if on_device else 1e-3 * n * n * 4 / 40e6      # 17 MB at 40 GB/s and above
     assert best[0.0] - upload < 0.5 * (best[1.0] - upload)
+
+
+@pytest.mark.parametrize("on_device", [False, True])
+def test_model_beyond_a_smaller_grid(on_device):
+    """With padding below 1 the grid is smaller than the image: an empty model
+    is taken as such, any other refused, also one whose only pixel lies outside
+    the grid."""
+    import torch
+    G, _, axes = setup("SphFunc", 64, 64, 1, 1, 0.5)
+    for at in (None, (0, 0), (32, 32)):
+        g = setup("SphFunc", 64, 64, 1, 1, 0.5)[1]
+        img = np.zeros((64, 64, 1, 1), dtype=np.float32, order="F")
+        if at:
+            img[at[0], at[1], 0, 0] = 1.0
+        give = torch.from_numpy(np.ascontiguousarray(img.transpose(3, 2, 1, 0))).cuda().permute(3, 2, 1, 0) \
+            if on_device else img
+        if at is None:
+            g.initialiseDegrid(axes, give)
+            assert g.isModelEmpty()
+        else:
+            with pytest.raises(G.AskapError):
+                g.initialiseDegrid(axes, give)

@@ -1399,6 +1399,19 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   const long long total = (long long)nx_ * ny_ * nplanes;
   const size_t gbytes = (size_t)ngrids() * total * sizeof(float2);
   cuda_check(grids_.ensure(gbytes), "alloc grids");
+  if (nx > nx_ || ny > ny_) {
+    // a grid smaller than the image (padding below 1) takes none but an empty
+    // model, empty also outside the grid, where the passes below do not look
+    std::vector<float> down(on_device ? in_total : 0);
+    if (on_device)
+      cuda_check(cudaMemcpy(down.data(), image, in_total * sizeof(float), cudaMemcpyDeviceToHost), "download model");
+    const float* h = on_device ? down.data() : image;
+    model_empty_ = std::none_of(h, h + in_total, [](float v) { return std::fabs(v) > 0.f; });
+    throw_if(!model_empty_, YG_ERR_CUDA, "initialiseDegrid: the padded grid is smaller than the image");
+    cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
+    sync();
+    return;
+  }
   // the model image on the device: the caller's, or an upload of it; the first
   // pass over it also tells whether it is empty
   cuda_check(img_tmp_.ensure(64 + (on_device ? 0 : in_total * sizeof(float))), "alloc");
@@ -1430,8 +1443,6 @@ void Gridder::initialise_degrid(const Axes& axes, int nx, int ny, int npol, int 
   model_empty_ = *flag.host == 0;
   if (model_empty_) cuda_check(cudaMemsetAsync(grids_.p, 0, gbytes, stream_), "memset");
   sync();
-  throw_if(!model_empty_ && (nx > nx_ || ny > ny_), YG_ERR_CUDA,
-           "initialiseDegrid: the padded grid is smaller than the image");
 }
 
 void Gridder::finalise_degrid() {
