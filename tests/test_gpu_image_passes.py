@@ -207,3 +207,21 @@ def test_model_beyond_a_smaller_grid(on_device):
         else:
             with pytest.raises(G.AskapError):
                 g.initialiseDegrid(axes, give)
+
+
+# sides that are powers of two fold the centring into the passes beside the FFT:
+# with screens, several planes and channels, extraction from a padded grid,
+# rectangular both ways
+ROLLED = [("WStack", 64, 64, 4, 1, 1.0), ("WStack", 128, 32, 2, 3, 1.0), ("SphFunc", 32, 128, 2, 3, 1.0),
+          ("SphFunc", 64, 32, 1, 1, 2.0), ("WStack", 32, 64, 3, 1, 2.0), ("SphFunc", 256, 512, 4, 1, 1.0)]
+
+
+@pytest.mark.parametrize("kind,nx,ny,npol,nchan,padding", ROLLED)
+def test_finalise_rolled(kind, nx, ny, npol, nchan, padding):
+    test_finalise(kind, nx, ny, npol, nchan, padding)
+
+
+@pytest.mark.parametrize("kind,nx,ny,npol,nchan,padding", ROLLED)
+@pytest.mark.parametrize("on_device", [False, True])
+def test_initialise_degrid_rolled(kind, nx, ny, npol, nchan, padding, on_device):
+    test_initialise_degrid(kind, nx, ny, npol, nchan, padding, on_device)
