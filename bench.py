@@ -71,7 +71,7 @@ def parse():
                          "config 1's field and CF support at a quarter of the grid memory)")
     ap.add_argument("--cell-arcsec", type=float, default=0.0, help="cell override (see --grid-nx)")
     ap.add_argument("--tile", type=int, default=0, help="uv tile side (0 = automatic)")
-    ap.add_argument("--variant", type=int, default=0, help="k_grid thread layout variant (0 = automatic)")
+    ap.add_argument("--variant", type=int, default=0, help="record order and thread layout of the grid kernels (0 = automatic)")
     ap.add_argument("--no-learned", action="store_true", help="skip the learned-CF leg")
     ap.add_argument("--no-tune", action="store_true", help="skip the autotuner")
     ap.add_argument("--learned-rows", type=float, default=0.01, help="fraction of the track the learned leg times")
@@ -524,17 +524,39 @@ def torch_index(a):
 # arms
 # --------------------------------------------------------------------------
 def kernel_names(variant, support):
-    """The grid and degrid kernels a pass runs for a k_grid variant: the
-    plane-major k_grid_pl with variant bit 64, else k_grid; k_degrid_r for
-    16-wide CFs unless variant bit 256 asks for k_degrid_t."""
+    """The layout families of a variant: k_grid_pl with variant bit 64, else
+    k_grid, whose CF-major records k_grid_cf grids too (grid_kernel says which
+    runs); k_degrid_r for 16-wide CFs unless variant bit 256 asks for
+    k_degrid_t."""
     v = variant or 1
     grid = "k_grid_pl" if v & 64 else "k_grid"
     degrid = "k_degrid_r" if (2 * support + 1 <= 16 and not v & 256) else "k_degrid_t"
     return grid, degrid
 
 
+def grid_kernel(variant, kind):
+    """The grid kernel that a pass runs: k_grid_pl with variant bit 64 and as
+    AWProject's automatic choice, k_grid_cf for the CF-major choice of the
+    others (CFs of one size, as the workloads here have), k_grid for the
+    CF-major layouts that are asked for."""
+    layout = variant & 255
+    if layout & 64 or (layout == 0 and kind == "AWProject"):
+        return "k_grid_pl"
+    return "k_grid_cf" if layout <= 1 else "k_grid"
+
+
+def smem_bytes_per_tap(name, npol):
+    """Bytes that one tap moves through the shared-memory pipe for all
+    polarisations together: the 8 B CF tap and, where a cell lies in shared
+    memory, its read-modify-write (16 B per polarisation; gridding) or its read
+    (8 B; degridding).  k_grid_pl keeps the sums in registers."""
+    if name.startswith("k_degrid"):
+        return 8.0 * npol + 8.0
+    return 8.0 if name == "k_grid_pl" else 16.0 * npol + 8.0
+
+
 def roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak, peak_kind, sm_hz, cf_bytes,
-             names=("k_grid", "k_degrid_t")):
+             names=("k_grid_cf", "k_degrid_t")):
     """Roofline of the dominant kernel (the grid pass's) and of the degrid kernel, per launch
     (one grid or degrid pass over the workload).  The binding roofline time is
     t_roof = max(algorithmic HBM bytes / measured HBM bandwidth,
@@ -569,8 +591,8 @@ def roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak,
                         "frac": round(nvalid_vis / npol * taps * smem_per_tap / smem_peak / t, 4) if t > 0 else 0.0}}
         return out
 
-    g = one(kgrid_ms, hbm_grid, 16.0 * npol + 8.0)
-    dg = one(kdeg_ms, hbm_degrid, 8.0 * npol + 8.0)
+    g = one(kgrid_ms, hbm_grid, smem_bytes_per_tap(names[0], npol))
+    dg = one(kdeg_ms, hbm_degrid, smem_bytes_per_tap(names[1], npol))
     traffic = kgrid_traffic(info, support, npol, names[0])
     return {"bound": g["bound"], "kernel": names[0], "achieved": g["fp32"]["achieved_tflops"],
             "peak": g["fp32"]["peak_tflops"], "peak_kind": "nominal FP32 (148 SMs x 128 lanes x 2 flops) at the "
@@ -590,10 +612,13 @@ def roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak,
 # polarisation x padded-tile cell, from single-kernel ncu captures of a small
 # case of config 1 (k_grid: the sorted records and visibilities read per
 # sample, the padded tiles written per item)
+# (k_grid_cf: a record, the weighted visibilities' sectors and the sample's
+# share of its segment's CF matrix, 739.8 MB read for 6.53e6 samples; tiles,
+# 191.9 MB written for 4271 items of 40^2 cells x 4)
 # (k_grid_pl: a record and the weighted visibilities' sector per sample, the
 # rest of the capture apportioned to the cells of the items' slots, cleared and
 # reduced into)
-TRAFFIC_RATES = {"k_grid": (48.9, 0.84 * 8), "k_grid_pl": (48.0, 51.2)}
+TRAFFIC_RATES = {"k_grid": (48.9, 0.84 * 8), "k_grid_cf": (113.3, 7.0), "k_grid_pl": (48.0, 51.2)}
 
 
 def kgrid_traffic(info, support, npol, name="k_grid"):
@@ -696,9 +721,9 @@ def run_b200(args, w):
     taps = (2 * support + 1) ** 2
     hbm_peak, peak_kind = peaks()
     sm_hz = (clk.summary().get("sm_mhz") or 1965.0) * 1e6
-    variant = args.variant or ((tune or {}).get("variant") or 0)   # 0: the CF-major default
+    variant = args.variant or ((tune or {}).get("variant") or 0)   # 0: the automatic choice
     roof = roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak, peak_kind, sm_hz,
-                    gg.cf_bytes(), kernel_names(variant, support))
+                    gg.cf_bytes(), (grid_kernel(variant, w["gridder"]), kernel_names(variant, support)[1]))
     line = {
         "metric": METRIC,
         "cf_form": "plain (tabulated CF)",
@@ -1239,7 +1264,7 @@ def run_beams(args, w):
                      "gpu_build_s_all_gridders": round(ms_cf / 1e3, 3),
                      "bytes_per_gridder": int(ncf * taps * 8),
                      "padded_bytes_per_gridder": int(ncf * ((2 * support + 1 + 15) // 16 * 16) ** 2 * 8)},
-        "binding": {"resource": "shared memory", "note": "k_grid and k_degrid_t, whole step",
+        "binding": {"resource": "shared memory", "note": "k_grid_pl and k_degrid_t, whole step",
                     "taps_per_s": round(2 * taps * nvis / (ms_step / 1e3), 1)},
         "clocks": clk.summary(),
         "gpu_launches": int(cyc.nodes() * args.steps),
