@@ -41,6 +41,7 @@ struct GridPlArgs {
 // groups that work on an item of n samples (a power of two up to groups):
 // every group has a slot of its own to clear and to sum, so one is worth
 // having for 128 samples and more
+constexpr int kMaxGroups = 4;
 __host__ __device__ __forceinline__ int item_groups(int n, int groups) {
   int g = 1;
   while (2 * g <= groups && n >= 256 * g) g *= 2;
@@ -717,9 +718,16 @@ __global__ void __launch_bounds__(544, 1) k_grid_cf(const __grid_constant__ Grid
 }
 
 // grid[cell] += sum over the slots whose padded tile covers the cell, in a
-// fixed order (neighbouring tiles, their items, their groups).  One CTA per
-// (grid plane / channel, tile), one thread per cell for all polarisations (a
-// slot keeps a cell's polarisations together).
+// fixed order (neighbouring tiles, their items, their groups).  One thread per
+// cell for all polarisations (a slot keeps a cell's polarisations together);
+// blockIdx.x is the (grid plane / channel, tile), blockIdx.y the CTA's share of
+// its cells.  Bound by latency where the items of a short track crowd into few
+// tiles: a cell's loads from consecutive items, and from an item's groups, do
+// not wait for one another, and several CTAs share a tile where there are few
+// (1.2e6 samples x 1 in 1296 items of 94^2 cells, 576 tiles: one slot per item
+// 0.79 ms in a loop of one load at a time, 0.23 with loads in flight, 0.074
+// shared; k_halo_sum of the same items 0.25.  Up to four slots per item: 1.03,
+// 0.92, 0.29).
 struct HaloPlArgs {
   const int* item_base;      // per tile: first item
   const int* nit;            // per tile: number of items
@@ -734,7 +742,22 @@ struct HaloPlArgs {
   long long slot;
 };
 
+// a cell's polarisations
 template <int NPOL>
+__device__ __forceinline__ void load_cell(const float2* __restrict__ s, float2 (&v)[NPOL]) {
+  if (NPOL == 1) {
+    v[0] = s[0];
+  } else {
+#pragma unroll
+    for (int p = 0; p < NPOL; p += 2) {
+      const float4 q = *reinterpret_cast<const float4*>(s + p);
+      v[p] = make_float2(q.x, q.y);
+      v[p + 1 < NPOL ? p + 1 : p] = make_float2(q.z, q.w);
+    }
+  }
+}
+
+template <int NPOL, bool GROUPS>
 __global__ void __launch_bounds__(256) k_halo_pl(const __grid_constant__ HaloPlArgs a) {
   const long long tid = blockIdx.x;               // over ngc * ntiles
   const long long gc = tid / a.ntiles;
@@ -754,7 +777,7 @@ __global__ void __launch_bounds__(256) k_halo_pl(const __grid_constant__ HaloPlA
   const int gind = (int)(gc / a.nchan_img), ichan = (int)(gc % a.nchan_img);
   const size_t plane_cells = (size_t)a.nx * a.ny;
   const int T = a.tile;
-  for (int c = threadIdx.x; c < T * T; c += blockDim.x) {
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < T * T; c += gridDim.y * blockDim.x) {
     const int x = tx * T + c % T, y = ty * T + c / T;
     if (x >= a.nx || y >= a.ny) continue;
     float2 sum[NPOL];
@@ -774,38 +797,41 @@ __global__ void __launch_bounds__(256) k_halo_pl(const __grid_constant__ HaloPlA
         const long long nt = gc * a.ntiles + ax + (long long)a.ntx * ay;
         const int b = a.item_base[nt];
         const int j0 = max(b, a.item0), j1 = min(b + a.nit[nt], a.item1);
-        for (int j = j0; j < j1; ++j) {
-          const int4 it = a.items[j];
-          const int G = item_groups(it.z - it.y, a.groups);
-          const float2* s = a.scratch + (size_t)(j - a.item0) * a.groups * a.slot +
-                            ((size_t)px + (size_t)a.P * py) * NPOL;
-          float2 isum[NPOL];                      // the item's groups first, then the items
-#pragma unroll
-          for (int p = 0; p < NPOL; ++p) isum[p] = make_float2(0.f, 0.f);
-          for (int g = 0; g < G; ++g, s += a.slot) {
+        hit = hit || j0 < j1;
+        const float2* s = a.scratch + (size_t)(j0 - a.item0) * a.groups * a.slot + ((size_t)px + (size_t)a.P * py) * NPOL;
+        if (!GROUPS) {
+#pragma unroll 4
+          for (int j = j0; j < j1; ++j, s += a.slot) {
             float2 v[NPOL];
-            if (NPOL == 1) {
-              v[0] = s[0];
-            } else {
-#pragma unroll
-              for (int p = 0; p < NPOL; p += 2) {
-                const float4 q = *reinterpret_cast<const float4*>(s + p);
-                v[p] = make_float2(q.x, q.y);
-                v[p + 1 < NPOL ? p + 1 : p] = make_float2(q.z, q.w);
-              }
-            }
+            load_cell<NPOL>(s, v);
 #pragma unroll
             for (int p = 0; p < NPOL; ++p) {
-              isum[p].x += v[p].x;
-              isum[p].y += v[p].y;
+              sum[p].x += v[p].x;
+              sum[p].y += v[p].y;
             }
           }
+        } else {
+#pragma unroll(NPOL == 4 ? 1 : 2)
+          for (int j = j0; j < j1; ++j, s += a.groups * a.slot) {
+            const int4 it = a.items[j];
+            const int G = item_groups(it.z - it.y, a.groups);
+            float2 v[kMaxGroups][NPOL], isum[NPOL];   // the item's groups first, then the items
 #pragma unroll
-          for (int p = 0; p < NPOL; ++p) {
-            sum[p].x += isum[p].x;
-            sum[p].y += isum[p].y;
+            for (int g = 0; g < kMaxGroups; ++g)
+              if (g < G) load_cell<NPOL>(s + g * a.slot, v[g]);
+#pragma unroll
+            for (int p = 0; p < NPOL; ++p) {
+              isum[p] = v[0][p];
+#pragma unroll
+              for (int g = 1; g < kMaxGroups; ++g) {
+                if (g >= G) continue;
+                isum[p].x += v[g][p].x;
+                isum[p].y += v[g][p].y;
+              }
+              sum[p].x += isum[p].x;
+              sum[p].y += isum[p].y;
+            }
           }
-          hit = true;
         }
       }
     }
@@ -859,7 +885,7 @@ Shape shape_for(int W, int npol, size_t block) {
   const int maxw = npol == 1 ? 12 : (s.sl <= 4 ? 8 : 7);
   s.parts = (wslots + s.sl * maxw - 1) / (s.sl * maxw);
   s.nw = (wslots + s.sl * s.parts - 1) / (s.sl * s.parts);
-  while (s.groups < 4 && 2 * s.groups * s.nw <= std::min(maxw, 8)) s.groups *= 2;
+  while (s.groups < kMaxGroups && 2 * s.groups * s.nw <= std::min(maxw, 8)) s.groups *= 2;
   const size_t fixed = block + 64 + fetch_bytes(npol), stage = stage_bytes(npol) + 16;
   const size_t budget = fixed + 2 * s.groups * stage <= kSmemTwo ? kSmemTwo : kSmemOne;
   s.nstages = fixed < budget ? (int)std::min<size_t>(16, (budget - fixed) / stage) / s.groups * s.groups : 0;
@@ -931,11 +957,20 @@ HaloPlArgs halo_args(const Plan& pl, const VisArgs& v, float2* grid, int nx, int
   return h;
 }
 
-int halo_sum(const HaloPlArgs& h, int npa, unsigned nblocks, cudaStream_t st) {
+template <int NPOL>
+void launch_halo(const HaloPlArgs& h, dim3 blocks, cudaStream_t st) {
+  if (h.groups > 1) k_halo_pl<NPOL, true><<<blocks, 256, 0, st>>>(h);
+  else k_halo_pl<NPOL, false><<<blocks, 256, 0, st>>>(h);
+}
+
+int halo_sum(const HaloPlArgs& h, int npa, unsigned ntiles, cudaStream_t st) {
+  // a few hundred large tiles would leave the chip idle: several CTAs share one
+  const unsigned share = std::max(1u, std::min({8u, 148u * 16 / ntiles, (unsigned)h.tile * h.tile / 512}));
+  const dim3 blocks(ntiles, share);
   switch (npa) {
-    case 1: k_halo_pl<1><<<nblocks, 256, 0, st>>>(h); break;
-    case 2: k_halo_pl<2><<<nblocks, 256, 0, st>>>(h); break;
-    default: k_halo_pl<4><<<nblocks, 256, 0, st>>>(h); break;
+    case 1: launch_halo<1>(h, blocks, st); break;
+    case 2: launch_halo<2>(h, blocks, st); break;
+    default: launch_halo<4>(h, blocks, st); break;
   }
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError() == cudaSuccess ? YG_OK : YG_ERR_CUDA;
