@@ -186,3 +186,37 @@ def test_slot_beyond_32_bits(kind, variant):
         with pytest.raises(G.AskapError) as e:
             g.grid(acc)
         assert e.value.code == 9
+
+
+def _kernels(run):
+    """Names of the grid kernels that run() launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in prof.key_averages())
+    return {k for k in ("k_grid<", "k_grid_cf<", "k_grid_pl<") if k in names}
+
+
+@pytest.mark.parametrize("support,npol,kernel", [
+    (19, 4, "k_grid_cf<"), (20, 1, "k_grid_cf<"), (21, 1, "k_grid<"), (21, 2, "k_grid_cf<"), (22, 3, "k_grid<"),
+    (22, 4, "k_grid_cf<"), (23, 1, "k_grid<"), (23, 2, "k_grid<"), (23, 4, "k_grid<"), (24, 1, "k_grid_cf<"),
+    (24, 4, "k_grid_cf<")])
+def test_cf_major_kernel_by_width(support, npol, kernel):
+    """CF-major passes take the faster of their two kernels (widths around 47,
+    where k_grid's padding is thin); the sums are the same bit for bit."""
+    from yandasoft_b200.gridder import Accessor
+    ds = _data(npol, 390 + support)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    out = []
+    for variant in (0, 2):
+        g = _wproject(support, 4, wmax=12000.0)
+        g.set_tile(48 if support < 24 else 56)
+        g.set_grid_variant(variant)
+        out.append(_grid(g, npol, lambda g: g.grid(acc)))
+        assert g.support()[0] == support
+        if variant == 0:
+            assert _kernels(lambda: g.grid(acc)) == {kernel}
+    assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])

@@ -79,6 +79,9 @@ int plan_learned_inputs(Plan& pl, const double* uvw, const double* freq, double 
                         int nchan_img, const double* wstack, double wnorm, cudaStream_t st);
 int grid_cf_buffer_bytes(int wpad);
 int grid_tile_for(int smax, int npol, bool varsup);
+// polarisations of one k_grid pass over a table at this tile side, its CFs
+// through the ring; 0: they do not fit
+int grid_ring_pols(const CFView& cf, int tile, int npol);
 int grid_tile_stride(int tile, int wpad, int smax, bool varsup);
 extern std::atomic<long long> g_kernel_launches;
 

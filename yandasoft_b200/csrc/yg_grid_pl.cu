@@ -849,6 +849,10 @@ __global__ void __launch_bounds__(256) k_halo_pl(const __grid_constant__ HaloPlA
   }
 }
 
+// a CF table of which L2 (126 MB) holds little beside the rest, and samples per
+// CF plane below which a tile holds hardly two of one matrix
+constexpr long long kBigTable = 32ll << 20, kSparsePlane = 4000;
+
 // Shared memory of a CTA, and what two CTAs of one SM may each take of it.
 constexpr size_t kSmemOne = 227 * 1024;
 constexpr size_t kSmemTwo = 113 * 1024;
@@ -1156,9 +1160,30 @@ cudaError_t launch_cf_any(const GridCfArgs& a, const CfShape& s, int nitems, cud
 
 }  // namespace
 
-bool grid_cf_takes(const CFView& cf, int P, int npol, int os) {
-  return !cf.varsup && cf.maxsize > 0 && (cf.maxsize & 1) && cf.maxsize <= 1023 && npol <= 4 &&
-         (long long)cf.ncf * (cf.maxsize * cf.maxsize + 1) <= 0x7fffffffll && cf_shape(cf.maxsize, P, npol, os > 8).npa;
+// Where k_grid (padded to Wp, CFs through a ring) is the faster of the two, per
+// launch, k_grid / k_grid_cf in ms:
+// - just below 48, where eight slots a thread or a polarisation per pass leave
+//   k_grid_cf short of warps and the padding is thin (1.8e6 samples, W 47: one
+//   polarisation 3.6 / 4.1, two 5.9 / 8.3, four 11.7 / 16.7; W 43, one 3.7 /
+//   4.1, but two, in one pass of four slots, 2.06 / 1.89 at 6e5 samples; from
+//   49 on k_grid pads to 64: W 49 6.3 / 4.6);
+// - tables of tens of MB with few samples per plane, whose segments are hardly
+//   longer than a sample (AWProject, 25344 matrices, 1.2e6 samples), at widths
+//   that fill k_grid's rows: W 13, two polarisations 1.16 / 1.32, four 1.41 /
+//   1.81, but one, with the sums after it, 1.69 / 1.58; W 31, one 2.26 / 2.48,
+//   two 3.02 / 3.30, but four 5.4 / 4.4; other widths the other way (W 29, two
+//   3.02 / 2.46; W 7, two 1.00 / 0.89).
+bool grid_cf_takes(const CFView& cf, int tile, int npol, int os, long long n) {
+  const int W = cf.maxsize;
+  if (cf.varsup || W <= 0 || (W & 1) == 0 || W > 1023 || npol > 4) return false;
+  const long long elems = (long long)cf.ncf * (W * W + 1);
+  if (elems > 0x7fffffffll) return false;
+  const CfShape s = cf_shape(W, tile + W - 1, npol, os > 8);
+  if (!s.npa) return false;
+  const bool sparse = elems * 8 > kBigTable && n < kSparsePlane * (cf.ncf / (os * os));
+  const bool thin = (s.sl >= 8 && W > 40 && W < 48) ||
+                    (sparse && ((W >= 13 && W < 16 && npol >= 2) || (W == 31 && npol <= 2)));
+  return !thin || grid_ring_pols(cf, tile, npol) == 0;
 }
 
 int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,

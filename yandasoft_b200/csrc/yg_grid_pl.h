@@ -14,9 +14,10 @@ int grid_pl_block(const CFView& cf, int os, int cf_mode, int npol);
 int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
                  DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1);
 
-// CF-major gridding with exact residue widths (k_grid_cf): whether it takes the
-// table at this padded tile side, and a pass over the plan's CF-major records.
-bool grid_cf_takes(const CFView& cf, int P, int npol, int os);
+// CF-major gridding with exact residue widths (k_grid_cf): whether it is to grid
+// n samples with the table at this tile side (k_grid grids the others), and a
+// pass over the plan's CF-major records.
+bool grid_cf_takes(const CFView& cf, int tile, int npol, int os, long long n);
 int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
                  int os, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
                  cudaEvent_t ev1);

@@ -936,8 +936,8 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // inverse of its own)
   const int layout = grid_layout() & 255;
   a.need_inv = a.keep_inv && (cf_form_ != 0 || (layout != 64 && !(layout & 32) &&
-                                                (layout != 1 || !grid_cf_takes(a.cf, a.tile + a.cf.maxsize - 1,
-                                                                               npol_, os_))));
+                                                (layout != 1 || !grid_cf_takes(a.cf, a.tile, npol_, os_,
+                                                                               dc.nrow * (long long)dc.nchan))));
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;

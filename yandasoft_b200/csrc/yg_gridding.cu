@@ -2219,6 +2219,13 @@ int grid_pols_per_pass(int npol, int Pg, int cfbuf, int nthr) {
   return 0;
 }
 
+int grid_ring_pols(const CFView& cf, int tile, int npol) {
+  if (!cf.pad || cf.wpad <= 0) return 0;
+  const int threads = grid_shape(cf.wpad).threads;
+  const int Pg = grid_tile_stride(tile, cf.wpad, (cf.maxsize - 1) / 2, cf.varsup != 0);
+  return threads ? grid_pols_per_pass(npol, Pg, (cf.wpad <= 16 ? 4 : 1) * grid_cf_buffer_bytes(cf.wpad), threads) : 0;
+}
+
 // Grids the samples of a plan onto `grid` (ngrid planes of (nx, ny, npol, nchan_img)).
 int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
               const SumwArgs& sw, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
@@ -2240,10 +2247,10 @@ int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, 
     return plan_grid_pl(pl, v, cf, grid, nx, ny, nchan_img, scratch, svis, err, st, ev0, ev1);
   }
   // the default CF-major layout: k_grid_cf (the same sums) where it takes the
-  // table; k_grid serves tables of several sizes, the learned CF and the
-  // layouts that are asked for
+  // table; k_grid serves the widths at which it is the faster, tables of
+  // several sizes, the learned CF and the layouts that are asked for
   if (!learned && !pl.grid_only && ((mode & 255) <= 1 || (mode & 255) == 64) && pl.nitems > 0 && cf.data && pl.keep_inv &&
-      grid_cf_takes(cf, pl.pad, v.npol, sw.os)) {
+      grid_cf_takes(cf, pl.tile, v.npol, sw.os, pl.nsamples)) {
     k_sum_weights<<<grid_dim(pl.nvalid, 256), 256, 0, st>>>(v, pl.rec.as<int4>(), pl.nvalid, sw, err);
     YG_COUNT_LAUNCH();
     YG_CUDA_TRY(cudaGetLastError());
