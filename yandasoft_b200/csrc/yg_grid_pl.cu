@@ -1186,6 +1186,31 @@ bool grid_cf_takes(const CFView& cf, int tile, int npol, int os, long long n) {
   return !thin || grid_ring_pols(cf, tile, npol) == 0;
 }
 
+// k_grid_pl lives from samples of a CF plane that share their footprint, and
+// from CF matrices that come out of L2.  Channel-rich tables on a few spread
+// integrations have neither (AWProject, 48 channels x 33 planes, 1.2e6 samples
+// of every 36th integration).  Grid passes, CF-major / plane-major in ms:
+// - tables beyond L2 (W 29: 170 MB): one polarisation 2.9 / 3.9, two 3.0 / 3.3;
+//   W 47 4.6 / 8.3 and 6.5 / 9.4; but where the CF-major kernel needs several
+//   passes and reads the table in each: W 51, two 10.5 / 10.1, four 20.6 / 14.3;
+//   W 39, four 8.5 / 7.7;
+// - tables within it, one polarisation: W 13 1.58 / 1.86, W 25 2.34 / 2.94, but
+//   W 7 1.45 / 1.11; two: W 13 1.96 / 1.45, W 25 2.84 / 2.88.
+// Consecutive integrations, or many samples to a plane, always gain (1e5
+// samples, 264 planes, W 47: 0.79 / 0.66, 1.29 / 0.68, 2.34 / 0.81 for one, two
+// and four polarisations; 1.8e6, 136 planes, W 57: 9.5 / 7.2, 15.9 / 8.3).
+bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n) {
+  constexpr long long kL2Table = 128ll << 20, kManyPlanes = 1000;
+  const int W = cf.maxsize;
+  const long long planes = cf.ncf / (os * os), table = (long long)cf.ncf * ((W * W + 1) & ~1) * 8;
+  if (n >= kSparsePlane * planes) return true;
+  const int pl_pols = pols_per_pass(W, npol, 0);
+  if (table <= kL2Table) return !(pl_pols == 1 && planes > kManyPlanes && W > 9);
+  const int cf_pols = grid_cf_takes(cf, tile, npol, os, n) ? cf_shape(W, tile + W - 1, npol, os > 8).npa
+                                                           : grid_ring_pols(cf, tile, npol);
+  return cf_pols < pl_pols;
+}
+
 int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
                  int os, DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0,
                  cudaEvent_t ev1) {

@@ -10,6 +10,10 @@ namespace yg {
 // number of matrices that the plane-major order treats as one CF plane.
 int grid_pl_block(const CFView& cf, int os, int cf_mode, int npol);
 
+// Whether plane-major records are the better choice for n samples, where the
+// order of a cell's sum is free (AWProject).
+bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n);
+
 // Grids the plane-major records of a plan (pl.rec_pos, pl.pl_fs).
 int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,
                  DevBuf& scratch, DevBuf& svis, DevError* err, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1);

@@ -797,24 +797,26 @@ bool Gridder::takes_planes() const {
   return cf_form_ == 0 && pad * pad * npol_ <= 0x7fffffffll && grid_pl_block(cf, os_, cf_mode(), npol_) != 0;
 }
 
-// The automatic choice: plane-major records (64) for AWProject where the
-// plane-major kernel takes the CF table, CF-major (1) otherwise.  The other
-// gridders' images are divided by the spheroidal, whose factors of 10^4 in the
-// corners turn the rounding of another order of a cell's sum into 1e-4 of the
-// image: their automatic choice keeps the CF-major order, so that an image
-// stays what it was bit for bit, and the plane-major order is theirs to ask for
-// or tune to.
-int Gridder::automatic_layout() const {
-  return kind_ == Kind::AWProject && !aw_taper_ && takes_planes() ? 64 : 1;
+// The automatic choice for n samples: plane-major records (64) for AWProject
+// where the plane-major kernel takes the CF table and is the better choice,
+// CF-major (1) otherwise.  The other gridders' images are divided by the
+// spheroidal, whose factors of 10^4 in the corners turn the rounding of another
+// order of a cell's sum into 1e-4 of the image: their automatic choice keeps
+// the CF-major order, so that an image stays what it was bit for bit, and the
+// plane-major order is theirs to ask for or tune to.
+int Gridder::automatic_layout(long long n) const {
+  if (kind_ != Kind::AWProject || aw_taper_ || !takes_planes()) return 1;
+  const CFView cf = cf_.view();
+  return grid_pl_better(cf, tile_for((cf.maxsize - 1) / 2, npol_), npol_, os_, n) ? 64 : 1;
 }
 
-// grid_variant() as plans are made by it and passes run by it (the records that
-// a plan happens to hold decide nothing): the automatic choice made, and with
-// bit 64 no other bit up to 128, or the CF-major layout where the plane-major
-// kernel does not take the CF table.
-int Gridder::grid_layout() const {
+// grid_variant() as plans of n samples are made by it and passes over them run
+// by it (the records that a plan happens to hold decide nothing): the automatic
+// choice made, and with bit 64 no other bit up to 128, or the CF-major layout
+// where the plane-major kernel does not take the CF table.
+int Gridder::grid_layout(long long n) const {
   const int v = grid_variant(), degrid = v & ~255;
-  if ((v & 255) == 0) return degrid | automatic_layout();
+  if ((v & 255) == 0) return degrid | automatic_layout(n);
   return v & 64 ? degrid | (takes_planes() ? 64 : 1) : v;
 }
 
@@ -856,7 +858,7 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   // 16-wide CFs grid with residue rows modulo their real width (exact rows)
   // unless a layout of several slots per thread was asked for
   const int wpad16 = ((2 * smax + 1) + 15) / 16 * 16;
-  const int variant = grid_layout();
+  const int variant = grid_layout(dc.nrow * (long long)dc.nchan);
   a.wy = (wpad16 == 16 && (variant & 15) <= 1 && exact_rows_) ? 2 * smax + 1 : 0;
   a.pl_fs = variant & 64 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
   a.pos_major = variant & 64 ? 2 : (variant & 32 ? 1 : 0);
@@ -934,17 +936,16 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // k_grid runs the layouts that are asked for, the learned CF and the tables
   // that neither of the other kernels takes (the position-major layout has an
   // inverse of its own)
-  const int layout = grid_layout() & 255;
+  const long long n = dc.nrow * (long long)dc.nchan;
+  const int layout = grid_layout(n) & 255;
   a.need_inv = a.keep_inv && (cf_form_ != 0 || (layout != 64 && !(layout & 32) &&
-                                                (layout != 1 || !grid_cf_takes(a.cf, a.tile, npol_, os_,
-                                                                               dc.nrow * (long long)dc.nchan))));
+                                                (layout != 1 || !grid_cf_takes(a.cf, a.tile, npol_, os_, n))));
   // samples per work item: enough items for ~8 per SM, never below 512
   int vmax = vmax_;
   TuneChoice tc;
   const bool tuned = tune_lookup(tune_class(), &tc);
   if (vmax <= 0 && tuned && tile_override_ <= 0) vmax = tc.vmax;
   if (vmax <= 0) {
-    const long long n = dc.nrow * (long long)dc.nchan;
     vmax = (int)std::min<long long>(1 << 20, std::max<long long>(512, n / (148 * 8)));
   }
   rc_check(plan_build(pl, a, vmax, err_.as<DevError>(), st), "binning");
@@ -1143,7 +1144,7 @@ void Gridder::grid_enqueue(const Chunk& dc, const Plan& pl, const float* mfs, cu
                     nsumw_rows_, nchan_};
   const LearnedCF lcf = learned_view_for(dc, const_cast<Plan&>(pl));
   rc_check(plan_grid(pl, v, cf_.view(), grids_.as<float2>(), nx_, ny_, nchan_, sw, scratch_, svis_,
-                     err_.as<DevError>(), st, k0, k1, grid_layout(), cf_form_ != 0 ? &lcf : nullptr),
+                     err_.as<DevError>(), st, k0, k1, grid_layout(pl.nsamples), cf_form_ != 0 ? &lcf : nullptr),
            "gridding");
   rc_check(plan_grid_carry(const_cast<Plan&>(pl), v, carry_.as<float2>(), st), "carry");
 }

@@ -169,7 +169,7 @@ class Gridder {
   int tile_for(int smax, int npol) const;
   TuneClass tune_class() const;
   int grid_variant() const;
-  int grid_layout() const;
+  int grid_layout(long long n) const;
   int items_vmax() const { return vmax_; }
   void set_vmax(int v) { vmax_ = v; }
   void sync();
@@ -206,7 +206,7 @@ class Gridder {
   void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
   int cf_mode() const;
   bool takes_planes() const;
-  int automatic_layout() const;
+  int automatic_layout(long long n) const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
   int corr_nx_ = 0, corr_ny_ = 0;      // shape that corr_d_ was made for
