@@ -534,15 +534,18 @@ def kernel_names(variant, support):
     return grid, degrid
 
 
-def grid_kernel(variant, kind):
-    """The grid kernel that a pass runs: k_grid_pl with variant bit 64 and as
-    AWProject's automatic choice, k_grid_cf for the CF-major choice of the
-    others (CFs of one size, as the workloads here have), k_grid for the
-    CF-major layouts that are asked for."""
-    layout = variant & 255
-    if layout & 64 or (layout == 0 and kind == "AWProject"):
+def grid_kernel(variant, support, npol):
+    """The grid kernel that a pass of the workloads here runs (CFs of one size;
+    AWProject's choice depends on its CF table and is not asked for): k_grid_pl
+    with variant bit 64; of the CF-major choice k_grid_cf, or k_grid at the
+    widths just below 48 that k_grid_cf grids one polarisation at a time; k_grid
+    for the CF-major layouts that are asked for."""
+    layout, width = variant & 255, 2 * support + 1
+    if layout & 64:
         return "k_grid_pl"
-    return "k_grid_cf" if layout <= 1 else "k_grid"
+    if layout > 1 or width == 47 or (width in (43, 45) and npol % 2):
+        return "k_grid"
+    return "k_grid_cf"
 
 
 def smem_bytes_per_tap(name, npol):
@@ -723,7 +726,7 @@ def run_b200(args, w):
     sm_hz = (clk.summary().get("sm_mhz") or 1965.0) * 1e6
     variant = args.variant or ((tune or {}).get("variant") or 0)   # 0: the automatic choice
     roof = roofline(w, d, info, support, npol, nvalid_vis, kgrid_ms, kdeg_ms, hbm_peak, peak_kind, sm_hz,
-                    gg.cf_bytes(), (grid_kernel(variant, w["gridder"]), kernel_names(variant, support)[1]))
+                    gg.cf_bytes(), (grid_kernel(variant, support, npol), kernel_names(variant, support)[1]))
     line = {
         "metric": METRIC,
         "cf_form": "plain (tabulated CF)",
@@ -1264,7 +1267,7 @@ def run_beams(args, w):
                      "gpu_build_s_all_gridders": round(ms_cf / 1e3, 3),
                      "bytes_per_gridder": int(ncf * taps * 8),
                      "padded_bytes_per_gridder": int(ncf * ((2 * support + 1 + 15) // 16 * 16) ** 2 * 8)},
-        "binding": {"resource": "shared memory", "note": "k_grid_pl and k_degrid_t, whole step",
+        "binding": {"resource": "shared memory", "note": "the grid kernel and k_degrid_t, whole step",
                     "taps_per_s": round(2 * taps * nvis / (ms_step / 1e3), 1)},
         "clocks": clk.summary(),
         "gpu_launches": int(cyc.nodes() * args.steps),

@@ -168,8 +168,8 @@ void yg_plan_destroy(yg_plan* plan);
 int yg_set_tile(yg_gridder* g, int32_t tile);      /* 0 = automatic */
 int yg_set_item_size(yg_gridder* g, int32_t vmax); /* samples per work item */
 /* Record order and thread layout of the grid kernels: 0 the default
- * (plane-major for AWProject, CF-major for the others), 1 CF-major, 2 and 3
- * halve / quarter the tap
+ * (plane-major for AWProject where its CF table and samples gain by it,
+ * CF-major for the others), 1 CF-major, 2 and 3 halve / quarter the tap
  * threads (each steps down twice / four times the rows); YG_ERR_UNSUPPORTED
  * at the next grid call when the CF width has no such layout.  Adding 16
  * keeps each thread's running tap sums in registers while consecutive

@@ -9,15 +9,14 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 
-@pytest.mark.parametrize("variant,kind,name", [
-    (0, "WStackWProject", "k_grid_cf"), (1, "WProject", "k_grid_cf"), (256, "WProject", "k_grid_cf"),
-    (2, "WProject", "k_grid"), (17, "WProject", "k_grid"), (49, "SphFunc", "k_grid"),
-    (64, "WProject", "k_grid_pl"), (193 | 512, "WProject", "k_grid_pl"), (0, "AWProject", "k_grid_pl"),
-    (1, "AWProject", "k_grid_cf")])
-def test_grid_kernel(variant, kind, name):
+@pytest.mark.parametrize("variant,support,npol,name", [
+    (0, 6, 4, "k_grid_cf"), (1, 19, 4, "k_grid_cf"), (256, 6, 1, "k_grid_cf"), (0, 23, 1, "k_grid"),
+    (1, 23, 2, "k_grid"), (0, 22, 2, "k_grid_cf"), (0, 22, 1, "k_grid"), (0, 24, 1, "k_grid_cf"), (2, 6, 4, "k_grid"),
+    (17, 6, 4, "k_grid"), (64, 6, 4, "k_grid_pl"), (193 | 512, 23, 1, "k_grid_pl")])
+def test_grid_kernel(variant, support, npol, name):
     import bench
-    assert bench.grid_kernel(variant, kind) == name
-    assert bench.kgrid_traffic({"tile": 32, "nvalid": 1000, "nitems": 10}, 6, 4, name) > 0
+    assert bench.grid_kernel(variant, support, npol) == name
+    assert bench.kgrid_traffic({"tile": 32, "nvalid": 1000, "nitems": 10}, support, npol, name) > 0
 
 
 def test_shared_memory_fraction():

@@ -207,6 +207,7 @@ def _kernels(run):
 def test_cf_major_kernel_by_width(support, npol, kernel):
     """CF-major passes take the faster of their two kernels (widths around 47,
     where k_grid's padding is thin); the sums are the same bit for bit."""
+    import bench
     from yandasoft_b200.gridder import Accessor
     ds = _data(npol, 390 + support)
     acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
@@ -219,6 +220,7 @@ def test_cf_major_kernel_by_width(support, npol, kernel):
         assert g.support()[0] == support
         if variant == 0:
             assert _kernels(lambda: g.grid(acc)) == {kernel}
+            assert bench.grid_kernel(variant, support, npol) + "<" == kernel    # the name that the bench prints
     assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
 
 
