@@ -168,3 +168,28 @@ def test_cf_major_full_ring(support, os_, npol, tile):
     assert np.abs(out[1][0]).max() > 0
     assert rel_l2(out[0][0], out[1][0]) < TOL
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("support,npol,tile,item", [(6, 3, 8, 0), (24, 4, 16, 0), (6, 3, 64, 300), (24, 4, 56, 100)])
+def test_halo_sums_of_passes(support, npol, tile, item):
+    """Several passes of polarisations with nearly all tiles empty (one halo sum
+    over all of them: 4096 and 1024 tiles, under 64 items) and with many items
+    to a tile (a sum per pass): the padded layout's sums, bit for bit."""
+    from yandasoft_b200 import simulate
+    from yandasoft_b200.gridder import Accessor, Axes
+    ds = simulate.make_dataset(duration_s=80.0 if item else 10.0, nchan=3 if item else 1, npol=npol, seed=7,
+                               diameter_m=600.0 if item else 60.0)
+    acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
+    out = []
+    for variant in (1, 2):
+        _, gg = _pair(support, 4)
+        gg.set_tile(tile)
+        if item:
+            gg.set_item_size(item)
+        gg.set_grid_variant(variant)
+        gg.initialiseGrid(Axes(CELL, CELL), (NX, NX, npol, 1))
+        plan = gg.plan(acc)
+        assert (plan.info()["nitems"] * 16 < (NX // tile) ** 2) == (item == 0)
+        gg.grid_plan(plan, acc)
+        out.append(np.stack(gg.grids()))
+    assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
