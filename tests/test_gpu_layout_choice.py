@@ -224,27 +224,38 @@ def test_cf_major_kernel_by_width(support, npol, kernel):
     assert np.abs(out[0]).max() > 0 and np.array_equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("support,npol,os_,nchan,kernel", [
-    (3, 1, 4, 48, "k_grid_pl<"), (6, 1, 4, 48, "k_grid_cf<"), (6, 2, 4, 48, "k_grid_pl<"), (6, 1, 4, 4, "k_grid_pl<"),
-    (6, 4, 8, 4, "k_grid_pl<"), (9, 2, 8, 48, "k_grid_cf<"), (7, 2, 8, 48, "k_grid<")])
-def test_awproject_order_by_table(support, npol, os_, nchan, kernel):
-    """AWProject's automatic choice: plane-major, but CF-major for channel-rich
-    tables on few samples (33 x 48 planes), beyond L2 (W 15 and 19 at oversample
-    8: 183 and 293 MB) or with one polarisation; either order's grid agrees with
-    the other's."""
+@pytest.mark.parametrize("support,npol,nchan,dt,kernel", [
+    (3, 1, 8, 1200.0, "k_grid_pl<"), (6, 1, 8, 1200.0, "k_grid_cf<"), (6, 1, 8, 0.5, "k_grid_pl<"),
+    (6, 2, 8, 1200.0, "k_grid_pl<"), (12, 4, 8, 1200.0, "k_grid_pl<"), (14, 2, 8, 1200.0, "k_grid_cf<"),
+    (14, 2, 8, 0.5, "k_grid_pl<"), (19, 1, 4, 1200.0, "k_grid_cf<"), (19, 1, 4, 0.5, "k_grid_pl<"),
+    (23, 2, 4, 1200.0, "k_grid<"), (23, 2, 4, 0.5, "k_grid_pl<"), (23, 4, 4, 1200.0, "k_grid_pl<")])
+def test_awproject_order_by_samples(support, npol, nchan, dt, kernel):
+    """AWProject's automatic choice: plane-major, but CF-major where the samples
+    of a CF plane hardly share footprints (integrations 20 minutes apart; eight
+    of half a second do) and the CFs are wide or the polarisation single, unless
+    the CF-major kernel needs several passes.  Through a plan and through
+    grid(), whose plans serve gridding only; either order's grid agrees with the
+    other's."""
     from yandasoft_b200 import simulate
     from yandasoft_b200.gridder import Accessor
-    ds = simulate.make_dataset(duration_s=20.0, nchan=nchan, npol=npol, seed=400, diameter_m=600.0)
+    ds = simulate.make_dataset(duration_s=8 * dt, dt_s=dt, nchan=nchan, npol=npol, seed=400, diameter_m=600.0)
     acc = Accessor(ds.uvw, ds.freq, ds.vis).to_device()
-    params = {"wmax": 2500.0, "nwplanes": 33, "oversample": os_, "maxsupport": 512, "limitsupport": support,
+    params = {"wmax": 5500.0, "nwplanes": 17, "oversample": 4, "maxsupport": 512, "limitsupport": support,
               "diameter": "12m", "blockage": "1m", "cutoff": 1e-3}
     out = []
     for variant in (0, 1, 64):
         g = make_pair("AWProject", params)[1]
         g.set_grid_variant(variant)
+        g.set_tile(48)
         out.append(_grid(g, npol, lambda g: g.grid(acc)))
         assert g.support()[0] == support
         if variant == 0:
             assert _kernels(lambda: g.grid(acc)) == {kernel}
+            plan = g.plan(acc)
+            assert _kernels(lambda: g.grid_plan(plan, acc)) == {kernel}
+            iu, iv, cfi, st = plan.samples(g, acc)
+            on = st == 3
+            cells = np.unique(np.stack([cfi[on] // 16, iu[on], iv[on]]), axis=1).shape[1]
+            print("%.2f samples per CF plane and cell" % (on.sum() / cells))
     assert np.array_equal(out[0], out[2] if kernel == "k_grid_pl<" else out[1])
     assert np.linalg.norm(out[1] - out[2]) <= 1e-5 * np.linalg.norm(out[1])

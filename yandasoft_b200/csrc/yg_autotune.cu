@@ -78,7 +78,9 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   // tried.
   std::vector<int> variants{1, 64, 17, 2};
   // the automatic choice comes first: the trial that default_ms reports
-  const int def_variant = automatic_layout(n);
+  Plan probe;
+  if (layout_asks(n)) bin(dc, probe);
+  const int def_variant = automatic_layout(n, probe.per_cell);
   std::stable_partition(variants.begin(), variants.end(), [&](int v) { return v == def_variant; });
   const int save_tile = tile_override_, save_vmax = vmax_, save_mode = grid_mode_;
   Chunk scratch_chunk = dc;

@@ -63,6 +63,9 @@ int cf_build_aw(CFCacheDev& cache, const AWCFParams& p, const std::vector<AWFeed
 
 // gridding entry points (yg_gridding.cu)
 int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t st);
+// bins the plan's samples (CF-major keys) and estimates pl.per_cell from a
+// hashed subset of them; waits for the answer
+int plan_samples_per_cell(Plan& pl, const BinArgs& a, DevError* err, cudaStream_t st);
 // Grids the samples of a plan and, when sw.sumw is set, adds their weights into
 // the sums of weights (one fused pass over the sorted samples).
 int plan_grid(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,

@@ -1190,29 +1190,36 @@ bool grid_cf_takes(const CFView& cf, int tile, int npol, int os, long long n) {
   return !thin || grid_ring_pols(cf, tile, npol) == 0;
 }
 
-// k_grid_pl lives from samples of a CF plane that share their footprint, and
-// from CF matrices that come out of L2.  Channel-rich tables on a few spread
-// integrations have neither (AWProject, 48 channels x 33 planes, 1.2e6 samples
-// of every 36th integration).  Grid passes, CF-major / plane-major in ms:
-// - tables beyond L2 (W 29: 170 MB): one polarisation 2.9 / 3.9, two 3.0 / 3.3;
-//   W 47 4.6 / 8.3 and 6.5 / 9.4; but where the CF-major kernel needs several
-//   passes and reads the table in each: W 51, two 10.5 / 10.1, four 20.6 / 14.3;
-//   W 39, four 8.5 / 7.7;
-// - tables within it, one polarisation: W 13 1.58 / 1.86, W 25 2.34 / 2.94, but
-//   W 7 1.45 / 1.11; two: W 13 1.96 / 1.45, W 25 2.84 / 2.88.
-// Consecutive integrations, or many samples to a plane, always gain (1e5
-// samples, 264 planes, W 47: 0.79 / 0.66, 1.29 / 0.68, 2.34 / 0.81 for one, two
-// and four polarisations; 1.8e6, 136 planes, W 57: 9.5 / 7.2, 15.9 / 8.3).
-bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n) {
-  constexpr long long kL2Table = 128ll << 20, kManyPlanes = 1000;
-  const int W = cf.maxsize;
-  const long long planes = cf.ncf / (os * os), table = (long long)cf.ncf * ((W * W + 1) & ~1) * 8;
-  if (n >= kSparsePlane * planes) return true;
-  const int pl_pols = pols_per_pass(W, npol, 0);
-  if (table <= kL2Table) return !(pl_pols == 1 && planes > kManyPlanes && W > 9);
+// k_grid_pl lives from samples of a CF plane that share their footprint; where
+// they do not, a move and mostly a matrix from beyond L1 per sample cost more
+// than the CF-major kernels' passes.  Grid passes, CF-major / plane-major in ms,
+// AWProject with 48 channels x 33 planes, 40 integrations of 5 s (1.2e6
+// samples), every 36th / 9th / 4th / 1st of a track, that is 1.05 / 1.58 / 3.0 /
+// 9.1 samples per plane and cell:
+//   W 47 to 37, one polarisation  4.6/8.3   3.2/4.0   3.1/3.0   3.0/2.1
+//               two               6.5/9.4   4.2/4.3   4.2/3.4   3.9/2.6
+//   W 29,       one               2.8/3.9   2.5/3.1   2.4/2.4   2.2/1.9
+//               two               3.0/3.3   2.7/2.7   2.8/2.1   2.5/1.7
+//               four              4.7/5.3   4.2/4.1   4.0/3.2   3.9/2.5
+//   W 25,       one               2.3/2.9   2.1/2.4   2.0/2.0   1.9/1.6
+//               two               2.8/2.8   2.6/2.3   2.4/1.9   2.3/1.5
+//   W 13,       one               1.6/1.9   1.4/1.6   1.3/1.4   1.3/1.2
+//               two               1.8/1.4   1.8/1.3   1.7/1.2   1.7/1.1
+// The size of the table hardly matters (24 channels, half of it: the same
+// ratios).  Where the CF-major kernel needs several passes it loses throughout
+// (W 39, four 8.5/7.6 to 7.3/3.3), as it does with many samples to a plane.
+bool grid_pl_asks(const CFView& cf, int tile, int npol, int os, long long n) {
+  const int W = cf.maxsize, pl_pols = pols_per_pass(W, npol, 0);
+  if (n >= kSparsePlane * (cf.ncf / (os * os))) return false;
+  if (pl_pols == 1) return W > 9;
+  if (W <= 25) return false;
   const int cf_pols = grid_cf_takes(cf, tile, npol, os, n) ? cf_shape(W, tile + W - 1, npol, os > 8).npa
                                                            : grid_ring_pols(cf, tile, npol);
-  return cf_pols < pl_pols;
+  return cf_pols >= pl_pols;
+}
+
+bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n, double per_cell) {
+  return !grid_pl_asks(cf, tile, npol, os, n) || per_cell >= (pols_per_pass(cf.maxsize, npol, 0) == 1 ? 3.0 : 2.0);
 }
 
 int plan_grid_cf(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,

@@ -10,9 +10,11 @@ namespace yg {
 // number of matrices that the plane-major order treats as one CF plane.
 int grid_pl_block(const CFView& cf, int os, int cf_mode, int npol);
 
-// Whether plane-major records are the better choice for n samples, where the
-// order of a cell's sum is free (AWProject).
-bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n);
+// Whether plane-major records are the better choice where the order of a cell's
+// sum is free (AWProject), and whether that depends on the samples per CF plane
+// and cell (plan_samples_per_cell).
+bool grid_pl_asks(const CFView& cf, int tile, int npol, int os, long long n);
+bool grid_pl_better(const CFView& cf, int tile, int npol, int os, long long n, double per_cell);
 
 // Grids the plane-major records of a plan (pl.rec_pos, pl.pl_fs).
 int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* grid, int nx, int ny, int nchan_img,

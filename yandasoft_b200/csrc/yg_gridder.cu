@@ -797,26 +797,33 @@ bool Gridder::takes_planes() const {
   return cf_form_ == 0 && pad * pad * npol_ <= 0x7fffffffll && grid_pl_block(cf, os_, cf_mode(), npol_) != 0;
 }
 
-// The automatic choice for n samples: plane-major records (64) for AWProject
-// where the plane-major kernel takes the CF table and is the better choice,
-// CF-major (1) otherwise.  The other gridders' images are divided by the
-// spheroidal, whose factors of 10^4 in the corners turn the rounding of another
-// order of a cell's sum into 1e-4 of the image: their automatic choice keeps
-// the CF-major order, so that an image stays what it was bit for bit, and the
-// plane-major order is theirs to ask for or tune to.
-int Gridder::automatic_layout(long long n) const {
+// The automatic choice for n samples, per_cell of them to a CF plane and cell
+// where layout_asks: plane-major records (64) for AWProject where the
+// plane-major kernel takes the CF table and is the better choice, CF-major (1)
+// otherwise.  The other gridders' images are divided by the spheroidal, whose
+// factors of 10^4 in the corners turn the rounding of another order of a cell's
+// sum into 1e-4 of the image: their automatic choice keeps the CF-major order,
+// so that an image stays what it was bit for bit, and the plane-major order is
+// theirs to ask for or tune to.
+int Gridder::automatic_layout(long long n, double per_cell) const {
   if (kind_ != Kind::AWProject || aw_taper_ || !takes_planes()) return 1;
   const CFView cf = cf_.view();
-  return grid_pl_better(cf, tile_for((cf.maxsize - 1) / 2, npol_), npol_, os_, n) ? 64 : 1;
+  return grid_pl_better(cf, tile_for((cf.maxsize - 1) / 2, npol_), npol_, os_, n, per_cell) ? 64 : 1;
 }
 
-// grid_variant() as plans of n samples are made by it and passes over them run
-// by it (the records that a plan happens to hold decide nothing): the automatic
-// choice made, and with bit 64 no other bit up to 128, or the CF-major layout
-// where the plane-major kernel does not take the CF table.
-int Gridder::grid_layout(long long n) const {
+bool Gridder::layout_asks(long long n) const {
+  if (kind_ != Kind::AWProject || aw_taper_ || !takes_planes()) return false;
+  const CFView cf = cf_.view();
+  return grid_pl_asks(cf, tile_for((cf.maxsize - 1) / 2, npol_), npol_, os_, n);
+}
+
+// grid_variant() as plans are made by it and passes over them run by it (the
+// records that a plan happens to hold decide nothing): the automatic choice
+// made, and with bit 64 no other bit up to 128, or the CF-major layout where
+// the plane-major kernel does not take the CF table.
+int Gridder::grid_layout(long long n, double per_cell) const {
   const int v = grid_variant(), degrid = v & ~255;
-  if ((v & 255) == 0) return degrid | automatic_layout(n);
+  if ((v & 255) == 0) return degrid | automatic_layout(n, per_cell);
   return v & 64 ? degrid | (takes_planes() ? 64 : 1) : v;
 }
 
@@ -827,7 +834,8 @@ int Gridder::tile_for(int smax, int npol) const {
   return grid_tile_for(smax, npol, cf_.view().varsup != 0);
 }
 
-void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const {
+void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok,
+                            double per_cell) const {
   a = BinArgs{};
   a.nrow = dc.nrow;
   a.nchan = dc.nchan;
@@ -858,7 +866,7 @@ void Gridder::fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, c
   // 16-wide CFs grid with residue rows modulo their real width (exact rows)
   // unless a layout of several slots per thread was asked for
   const int wpad16 = ((2 * smax + 1) + 15) / 16 * 16;
-  const int variant = grid_layout(dc.nrow * (long long)dc.nchan);
+  const int variant = grid_layout(dc.nrow * (long long)dc.nchan, per_cell);
   a.wy = (wpad16 == 16 && (variant & 15) <= 1 && exact_rows_) ? 2 * smax + 1 : 0;
   a.pl_fs = variant & 64 ? grid_pl_block(a.cf, os_, a.cf_mode, dc.npol) : 0;
   a.pos_major = variant & 64 ? 2 : (variant & 32 ? 1 : 0);
@@ -927,8 +935,17 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
     cuda_check(cudaMemcpyAsync(rowok_d_.p, rows.data(), rows.size(), cudaMemcpyHostToDevice, st), "up");
     row_ok = rowok_d_.as<uint8_t>();
   }
+  const long long n = dc.nrow * (long long)dc.nchan;
   BinArgs a;
-  fill_bin_args(a, dc, pl.chanmap.as<int>(), row_ok);
+  pl.per_cell = 0;
+  int binned = 0;
+  if (use != PLAN_DEGRID && layout_asks(n)) {
+    fill_bin_args(a, dc, pl.chanmap.as<int>(), row_ok);
+    rc_check(plan_samples_per_cell(pl, a, err_.as<DevError>(), st), "binning");
+    binned = 1;
+  }
+  fill_bin_args(a, dc, pl.chanmap.as<int>(), row_ok, pl.per_cell);
+  a.binned = binned;
   if (use == PLAN_DEGRID) a.pos_major = 0;
   // a gridding-only plan for the plane-major kernel sorts once, by its key
   a.key_planes = (use == PLAN_GRID && a.pos_major == 2) ? 1 : 0;
@@ -936,8 +953,7 @@ void Gridder::bin(const Chunk& dc, Plan& pl, cudaStream_t st, int use) {
   // k_grid runs the layouts that are asked for, the learned CF and the tables
   // that neither of the other kernels takes (the position-major layout has an
   // inverse of its own)
-  const long long n = dc.nrow * (long long)dc.nchan;
-  const int layout = grid_layout(n) & 255;
+  const int layout = grid_layout(n, pl.per_cell) & 255;
   a.need_inv = a.keep_inv && (cf_form_ != 0 || (layout != 64 && !(layout & 32) &&
                                                 (layout != 1 || !grid_cf_takes(a.cf, a.tile, npol_, os_, n))));
   // samples per work item: enough items for ~8 per SM, never below 512
@@ -1144,7 +1160,7 @@ void Gridder::grid_enqueue(const Chunk& dc, const Plan& pl, const float* mfs, cu
                     nsumw_rows_, nchan_};
   const LearnedCF lcf = learned_view_for(dc, const_cast<Plan&>(pl));
   rc_check(plan_grid(pl, v, cf_.view(), grids_.as<float2>(), nx_, ny_, nchan_, sw, scratch_, svis_,
-                     err_.as<DevError>(), st, k0, k1, grid_layout(pl.nsamples), cf_form_ != 0 ? &lcf : nullptr),
+                     err_.as<DevError>(), st, k0, k1, grid_layout(pl.nsamples, pl.per_cell), cf_form_ != 0 ? &lcf : nullptr),
            "gridding");
   rc_check(plan_grid_carry(const_cast<Plan&>(pl), v, carry_.as<float2>(), st), "carry");
 }

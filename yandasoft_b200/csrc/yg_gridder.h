@@ -169,7 +169,7 @@ class Gridder {
   int tile_for(int smax, int npol) const;
   TuneClass tune_class() const;
   int grid_variant() const;
-  int grid_layout(long long n) const;
+  int grid_layout(long long n, double per_cell) const;
   int items_vmax() const { return vmax_; }
   void set_vmax(int v) { vmax_ = v; }
   void sync();
@@ -203,10 +203,12 @@ class Gridder {
   void check_error(cudaStream_t st = nullptr);
   void upload_chunk(const Chunk& c, Chunk& dc, bool need_vis, bool vis_writable);
   std::vector<int> chan_map(const double* freq_host, int nchan) const;
-  void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok) const;
+  void fill_bin_args(BinArgs& a, const Chunk& dc, const int* dchan_map, const uint8_t* row_ok,
+                     double per_cell = 0) const;
   int cf_mode() const;
   bool takes_planes() const;
-  int automatic_layout(long long n) const;
+  int automatic_layout(long long n, double per_cell) const;
+  bool layout_asks(long long n) const;
   double wterm_cf(int plane) const;
   void prepare_corrections();
   int corr_nx_ = 0, corr_ny_ = 0;      // shape that corr_d_ was made for

@@ -1818,6 +1818,85 @@ static int inverse_for_pass(const Plan& plan, cudaStream_t st) {
   return YG_OK;
 }
 
+static int bin_samples(Plan& pl, const BinArgs& a, DevError* err, cudaStream_t st) {
+  const long long n = a.nrow * (long long)a.nchan;
+  YG_CUDA_TRY(pl.key.ensure(n * 8));
+  YG_CUDA_TRY(pl.key_alt.ensure(n * 8));
+  YG_CUDA_TRY(pl.val.ensure(n * 4));
+  YG_CUDA_TRY(pl.val_alt.ensure(n * 4));
+  YG_CUDA_TRY(pl.pos.ensure(n * 4));
+  YG_CUDA_TRY(pl.cfi.ensure(n * 4));
+  YG_CUDA_TRY(pl.status.ensure(n));
+  k_bin<<<grid_dim(n, 256), 256, 0, st>>>(a, pl.key.as<unsigned long long>(), pl.val.as<unsigned int>(),
+                                          pl.pos.as<unsigned int>(), pl.cfi.as<int>(),
+                                          pl.status.as<unsigned char>(), err);
+  YG_COUNT_LAUNCH();
+  YG_CUDA_TRY(cudaGetLastError());
+  return YG_OK;
+}
+
+// Counts the on-grid samples whose (CF plane, cell) hashes into a subset of one
+// in `mask` + 1, and the distinct ones among them, in a hash table of kDistinct
+// entries (linear probing; the subset fills half of it at most, so that no
+// probe comes near its limit).  All samples of a cell fall into the subset or
+// none, so counts[0] / counts[1] estimates the samples per plane and cell.  The
+// hash is the finaliser of SplitMix64 (Steele, Lea and Flood 2014).
+constexpr int kDistinct = 1 << 16;
+
+__global__ void k_distinct(const unsigned char* __restrict__ status, const unsigned int* __restrict__ pos,
+                           const int* __restrict__ cfi, long long n, int os2, unsigned mask,
+                           unsigned long long* __restrict__ table, int* __restrict__ counts) {
+  int seen = 0, fresh = 0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    if (status[i] != 3) continue;
+    const unsigned long long key = ((unsigned long long)(unsigned)(cfi[i] / os2) << 32) | pos[i];
+    unsigned long long h = key + 0x9e3779b97f4a7c15ull;
+    h = (h ^ (h >> 30)) * 0xbf58476d1ce4e5b9ull;
+    h = (h ^ (h >> 27)) * 0x94d049bb133111ebull;
+    h ^= h >> 31;
+    if ((unsigned)h & mask) continue;
+    ++seen;
+    unsigned at = (unsigned)(h >> 32) & (kDistinct - 1);
+    for (int probe = 0; probe < 256; ++probe, at = (at + 1) & (kDistinct - 1)) {
+      const unsigned long long was = atomicCAS(&table[at], ~0ull, key);
+      if (was == ~0ull) ++fresh;
+      if (was == ~0ull || was == key) break;
+    }
+  }
+  seen = __reduce_add_sync(0xffffffffu, seen);
+  fresh = __reduce_add_sync(0xffffffffu, fresh);
+  if ((threadIdx.x & 31) == 0 && seen) {
+    atomicAdd(&counts[0], seen);
+    atomicAdd(&counts[1], fresh);
+  }
+}
+
+int plan_samples_per_cell(Plan& pl, const BinArgs& a, DevError* err, cudaStream_t st) {
+  const long long n = a.nrow * (long long)a.nchan;
+  pl.per_cell = 0;
+  if (n == 0 || n >= (1ll << 31)) return YG_OK;
+  const int rc = bin_samples(pl, a, err, st);
+  if (rc) return rc;
+  const size_t table_bytes = (size_t)kDistinct * 8;
+  YG_CUDA_TRY(pl.distinct.ensure(table_bytes + 2 * sizeof(int)));
+  YG_CUDA_TRY(pl.info_h.ensure(16));
+  int* counts = reinterpret_cast<int*>(pl.distinct.as<unsigned char>() + table_bytes);
+  YG_CUDA_TRY(cudaMemsetAsync(pl.distinct.p, 0xff, table_bytes, st));
+  YG_CUDA_TRY(cudaMemsetAsync(counts, 0, 2 * sizeof(int), st));
+  unsigned mask = 0;
+  while (n / (mask + 1) > kDistinct / 2) mask = 2 * mask + 1;
+  k_distinct<<<grid_dim(n, 256), 256, 0, st>>>(pl.status.as<unsigned char>(), pl.pos.as<unsigned int>(),
+                                               pl.cfi.as<int>(), n, a.os * a.os, mask,
+                                               pl.distinct.as<unsigned long long>(), counts);
+  YG_COUNT_LAUNCH();
+  YG_CUDA_TRY(cudaGetLastError());
+  YG_CUDA_TRY(cudaMemcpyAsync(pl.info_h.p, counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  YG_CUDA_TRY(cudaStreamSynchronize(st));
+  const int seen = pl.info_h.as<volatile int>()[0], fresh = pl.info_h.as<volatile int>()[1];
+  pl.per_cell = fresh > 0 ? (double)seen / fresh : 0;
+  return YG_OK;
+}
+
 // Bins one chunk: fills plan (sorted ids, tile table, work items).
 int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t st) {
   const long long n = a.nrow * (long long)a.nchan;
@@ -1847,18 +1926,10 @@ int plan_build(Plan& pl, const BinArgs& a, int vmax, DevError* err, cudaStream_t
     return YG_OK;
   }
   if (n >= (1ll << 31)) return YG_ERR_ARG;  // sort sizes and tile offsets are int
-  YG_CUDA_TRY(pl.key.ensure(n * 8));
-  YG_CUDA_TRY(pl.key_alt.ensure(n * 8));
-  YG_CUDA_TRY(pl.val.ensure(n * 4));
-  YG_CUDA_TRY(pl.val_alt.ensure(n * 4));
-  YG_CUDA_TRY(pl.pos.ensure(n * 4));
-  YG_CUDA_TRY(pl.cfi.ensure(n * 4));
-  YG_CUDA_TRY(pl.status.ensure(n));
-  k_bin<<<grid_dim(n, 256), 256, 0, st>>>(a, pl.key.as<unsigned long long>(), pl.val.as<unsigned int>(),
-                                          pl.pos.as<unsigned int>(), pl.cfi.as<int>(),
-                                          pl.status.as<unsigned char>(), err);
-  YG_COUNT_LAUNCH();
-  YG_CUDA_TRY(cudaGetLastError());
+  if (!a.binned || a.key_planes) {
+    const int rc = bin_samples(pl, a, err, st);
+    if (rc) return rc;
+  }
   // radix sort over the bits that keys use (the invalid key is one past the
   // largest valid key, so it sorts last)
   const int end_bit = std::min(64, ceil_log2(a.invalid_key + 1));

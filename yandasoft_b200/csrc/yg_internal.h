@@ -124,6 +124,7 @@ struct BinArgs {
   int key_planes;          // a plan for gridding only: sort once, by the plane-major key (pos_major 2)
   int keep_inv;            // the CF-major records may be gridded: their inverse permutation can be built later
   int need_inv;            // it is built with the plan: the layout and the CF table are k_grid's
+  int binned;              // plan_samples_per_cell has binned the plan's samples with these arguments
   unsigned long long invalid_key;  // one past the largest valid key
   CFView cf;
 };
@@ -157,6 +158,8 @@ struct Plan {
   bool inv_ready = false, inv_pos_ready = false;   // inv / inv_pos are built
   bool keep_inv = false;        // inv may be built when a pass first needs it
   std::mutex inv_mutex;         // held by the pass that builds it
+  DevBuf distinct;              // plan_samples_per_cell: hash table of (CF plane, cell) and two counts
+  double per_cell = 0;          // samples per CF plane and footprint, 0: not asked for
   int pos_mode = 0;             // its order: 1 position then CF index; 2 CF plane, position, offset
   int pl_fs = 0;                // plane-major records: grid_pl_block of their CF table
   DevBuf ext;                   // continuous learned CF: per sorted sample (ru, rv, w, 0)
