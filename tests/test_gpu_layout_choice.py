@@ -197,6 +197,8 @@ def _kernels(run):
         run()
         torch.cuda.synchronize()
     names = " ".join(e.key for e in prof.key_averages())
+    if "k_" not in names:
+        pytest.skip("the profiler traced no kernels")
     return {k for k in ("k_grid<", "k_grid_cf<", "k_grid_pl<") if k in names}
 
 
@@ -225,16 +227,17 @@ def test_cf_major_kernel_by_width(support, npol, kernel):
 
 
 @pytest.mark.parametrize("support,npol,nchan,dt,kernel", [
-    (3, 1, 8, 1200.0, "k_grid_pl<"), (6, 1, 8, 1200.0, "k_grid_cf<"), (6, 1, 8, 0.5, "k_grid_pl<"),
-    (6, 2, 8, 1200.0, "k_grid_pl<"), (12, 4, 8, 1200.0, "k_grid_pl<"), (14, 2, 8, 1200.0, "k_grid_cf<"),
-    (14, 2, 8, 0.5, "k_grid_pl<"), (19, 1, 4, 1200.0, "k_grid_cf<"), (19, 1, 4, 0.5, "k_grid_pl<"),
-    (23, 2, 4, 1200.0, "k_grid<"), (23, 2, 4, 0.5, "k_grid_pl<"), (23, 4, 4, 1200.0, "k_grid_pl<")])
+    (3, 1, 16, 1200.0, "k_grid_pl<"), (6, 1, 16, 1200.0, "k_grid_cf<"), (6, 1, 16, 0.5, "k_grid_pl<"),
+    (6, 1, 8, 1200.0, "k_grid_pl<"), (6, 2, 16, 1200.0, "k_grid_pl<"), (12, 4, 16, 1200.0, "k_grid_pl<"),
+    (14, 2, 16, 1200.0, "k_grid_cf<"), (14, 2, 16, 0.5, "k_grid_pl<"), (19, 1, 16, 1200.0, "k_grid_cf<"),
+    (19, 1, 16, 0.5, "k_grid_pl<"), (23, 2, 16, 1200.0, "k_grid<"), (23, 2, 16, 0.5, "k_grid_pl<"),
+    (23, 4, 16, 1200.0, "k_grid_pl<")])
 def test_awproject_order_by_samples(support, npol, nchan, dt, kernel):
     """AWProject's automatic choice: plane-major, but CF-major where the samples
     of a CF plane hardly share footprints (integrations 20 minutes apart; eight
     of half a second do) and the CFs are wide or the polarisation single, unless
-    the CF-major kernel needs several passes.  Through a plan and through
-    grid(), whose plans serve gridding only; either order's grid agrees with the
+    the CF-major kernel needs several passes or the chunk is small.  Through a
+    plan and through grid(), whose plans serve gridding only; either order's grid agrees with the
     other's."""
     from yandasoft_b200 import simulate
     from yandasoft_b200.gridder import Accessor

@@ -72,10 +72,9 @@ TuneReport Gridder::autotune(const Chunk& dc, int max_trials) {
   for (int v : {def_vmax / 4, def_vmax * 4})
     if (v >= 128 && v <= (1 << 20)) vmaxes.push_back(v);
   // record orders and thread layouts: the CF-major kernel (1), the plane-major
-  // kernel (64), half the CF-major kernel's threads (2) and its tap sums in
-  // registers (17).  Position-major records with taps
-  // through L2 (32) measured slower on the benchmark workloads and are not
-  // tried.
+  // kernel (64), k_grid with its tap sums in registers (17) and with half its
+  // threads (2).  Position-major records with taps through L2 (32) measured
+  // slower on the benchmark workloads and are not tried.
   std::vector<int> variants{1, 64, 17, 2};
   // the automatic choice comes first: the trial that default_ms reports
   Plan probe;

@@ -60,9 +60,7 @@ CFView CFCacheDev::view() const {
   v.ncf = ncf;
   v.noffsets = noffsets;
   v.maxsize = maxsize;
-  v.varsup = 0;
-  for (int sz : h_size)
-    if (sz != 0 && sz != maxsize) v.varsup = 1;
+  v.varsup = varsup;
   v.pad = pad.p ? pad.as<float2>() : nullptr;
   v.wpad = wpad;
   return v;
@@ -107,6 +105,7 @@ int CFCacheDev::layout(const std::vector<int>& sizes, const std::vector<int2>& o
     tot += (long long)sizes[i] * sizes[i];
     maxsize = std::max(maxsize, sizes[i]);
   }
+  varsup = std::any_of(sizes.begin(), sizes.end(), [&](int sz) { return sz != 0 && sz != maxsize; }) ? 1 : 0;
   total = tot;
   h_offsets = offs;
   noffsets = (int)offs.size();

@@ -12,6 +12,7 @@ struct CFCacheDev {
   int ncf = 0;
   int noffsets = 0;
   int maxsize = 0;
+  int varsup = 0;           // 1 when CF sizes differ (set with the layout: a view is taken many times per call)
   int support = 0;          // itsSupport
   long long total = 0;      // complex elements
   std::vector<int> h_size;

@@ -1037,8 +1037,9 @@ int plan_grid_pl(const Plan& pl, const VisArgs& v, const CFView& cf, float2* gri
   g.block_bytes = (int)block;
   g.slot = ((long long)P * P * npa + 1) & ~1ll;
   g.err = err;
-  // scratch for at most kScratch bytes of slots at a time: launches over
-  // consecutive items, each followed by its halo sum
+  // scratch for kScratch bytes of slots at a time, or for 1184 items (eight per
+  // SM) where those are more: launches over consecutive items, each followed by
+  // its halo sum
   constexpr size_t kScratch = (size_t)4 << 30;
   const size_t per_item = (size_t)s.groups * g.slot * sizeof(float2);
   const int batch = (int)std::min<long long>(pl.nitems, std::max<long long>(1184, (long long)(kScratch / per_item)));
@@ -1210,7 +1211,9 @@ bool grid_cf_takes(const CFView& cf, int tile, int npol, int os, long long n) {
 // (W 39, four 8.5/7.6 to 7.3/3.3), as it does with many samples to a plane.
 bool grid_pl_asks(const CFView& cf, int tile, int npol, int os, long long n) {
   const int W = cf.maxsize, pl_pols = pols_per_pass(W, npol, 0);
-  if (n >= kSparsePlane * (cf.ncf / (os * os))) return false;
+  // (asking costs 30 us: 15,000 samples, 0.49 -> 0.52 ms per grid call, to
+  // choose between kernels of 0.08 ms)
+  if (n < (1 << 16) || n >= kSparsePlane * (cf.ncf / (os * os))) return false;
   if (pl_pols == 1) return W > 9;
   if (W <= 25) return false;
   const int cf_pols = grid_cf_takes(cf, tile, npol, os, n) ? cf_shape(W, tile + W - 1, npol, os > 8).npa

@@ -18,8 +18,8 @@
 //                  the cells of a fixed residue class (x mod W, y mod W), so no
 //                  two threads ever touch the same cell (no atomics); its
 //                  weighted visibilities come from k_gather_cube.
-//   k_grid_cf      (yg_grid_pl.cu) the same sums with exact CF widths: the
-//                  default for CF-major records.
+//   k_grid_cf      (yg_grid_pl.cu) the same sums with exact CF widths, where
+//                  that is the faster (grid_cf_takes).
 //   k_grid_pl      (yg_grid_pl.cu) over plane-major records, running sums in
 //                  registers.
 //   k_halo_sum     each output tile adds, in a fixed order, the overlapping
@@ -1836,15 +1836,13 @@ static int bin_samples(Plan& pl, const BinArgs& a, DevError* err, cudaStream_t s
 }
 
 // Counts the on-grid samples whose (CF plane, cell) hashes into a subset of one
-// in `mask` + 1, and the distinct ones among them, in a hash table of kDistinct
-// entries (linear probing; the subset fills half of it at most, so that no
-// probe comes near its limit).  All samples of a cell fall into the subset or
-// none, so counts[0] / counts[1] estimates the samples per plane and cell.  The
-// hash is the finaliser of SplitMix64 (Steele, Lea and Flood 2014).
-constexpr int kDistinct = 1 << 16;
-
+// in `mask` + 1, and the distinct ones among them, in a hash table (linear
+// probing; the subset fills half of it at most, so that no probe comes near its
+// limit).  All samples of a cell fall into the subset or none, so counts[0] /
+// counts[1] estimates the samples per plane and cell.  The hash is the finaliser
+// of SplitMix64 (Steele, Lea and Flood 2014).
 __global__ void k_distinct(const unsigned char* __restrict__ status, const unsigned int* __restrict__ pos,
-                           const int* __restrict__ cfi, long long n, int os2, unsigned mask,
+                           const int* __restrict__ cfi, long long n, int os2, unsigned mask, unsigned entries,
                            unsigned long long* __restrict__ table, int* __restrict__ counts) {
   int seen = 0, fresh = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -1856,8 +1854,8 @@ __global__ void k_distinct(const unsigned char* __restrict__ status, const unsig
     h ^= h >> 31;
     if ((unsigned)h & mask) continue;
     ++seen;
-    unsigned at = (unsigned)(h >> 32) & (kDistinct - 1);
-    for (int probe = 0; probe < 256; ++probe, at = (at + 1) & (kDistinct - 1)) {
+    unsigned at = (unsigned)(h >> 32) & (entries - 1);
+    for (int probe = 0; probe < 256; ++probe, at = (at + 1) & (entries - 1)) {
       const unsigned long long was = atomicCAS(&table[at], ~0ull, key);
       if (was == ~0ull) ++fresh;
       if (was == ~0ull || was == key) break;
@@ -1877,20 +1875,22 @@ int plan_samples_per_cell(Plan& pl, const BinArgs& a, DevError* err, cudaStream_
   if (n == 0 || n >= (1ll << 31)) return YG_OK;
   const int rc = bin_samples(pl, a, err, st);
   if (rc) return rc;
-  const size_t table_bytes = (size_t)kDistinct * 8;
-  YG_CUDA_TRY(pl.distinct.ensure(table_bytes + 2 * sizeof(int)));
+  // the table in the sort's alternate keys, at most one entry per sample (with
+  // 512 KB of its own an image of 15,000 samples took 4.4 ms instead of 3.7: the
+  // allocations of later calls' temporary buffers became slower)
+  YG_CUDA_TRY(pl.nvalid_d.ensure(16));
   YG_CUDA_TRY(pl.info_h.ensure(16));
-  int* counts = reinterpret_cast<int*>(pl.distinct.as<unsigned char>() + table_bytes);
-  YG_CUDA_TRY(cudaMemsetAsync(pl.distinct.p, 0xff, table_bytes, st));
-  YG_CUDA_TRY(cudaMemsetAsync(counts, 0, 2 * sizeof(int), st));
-  unsigned mask = 0;
-  while (n / (mask + 1) > kDistinct / 2) mask = 2 * mask + 1;
+  unsigned entries = 1, mask = 0;
+  while (entries < (1u << 16) && 2ll * entries <= n) entries *= 2;
+  while (n / (mask + 1) > entries / 2) mask = 2 * mask + 1;
+  YG_CUDA_TRY(cudaMemsetAsync(pl.key_alt.p, 0xff, (size_t)entries * 8, st));
+  YG_CUDA_TRY(cudaMemsetAsync(pl.nvalid_d.p, 0, 16, st));
   k_distinct<<<grid_dim(n, 256), 256, 0, st>>>(pl.status.as<unsigned char>(), pl.pos.as<unsigned int>(),
-                                               pl.cfi.as<int>(), n, a.os * a.os, mask,
-                                               pl.distinct.as<unsigned long long>(), counts);
+                                               pl.cfi.as<int>(), n, a.os * a.os, mask, entries,
+                                               pl.key_alt.as<unsigned long long>(), pl.nvalid_d.as<int>());
   YG_COUNT_LAUNCH();
   YG_CUDA_TRY(cudaGetLastError());
-  YG_CUDA_TRY(cudaMemcpyAsync(pl.info_h.p, counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  YG_CUDA_TRY(cudaMemcpyAsync(pl.info_h.p, pl.nvalid_d.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   YG_CUDA_TRY(cudaStreamSynchronize(st));
   const int seen = pl.info_h.as<volatile int>()[0], fresh = pl.info_h.as<volatile int>()[1];
   pl.per_cell = fresh > 0 ? (double)seen / fresh : 0;

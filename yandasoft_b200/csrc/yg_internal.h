@@ -158,7 +158,6 @@ struct Plan {
   bool inv_ready = false, inv_pos_ready = false;   // inv / inv_pos are built
   bool keep_inv = false;        // inv may be built when a pass first needs it
   std::mutex inv_mutex;         // held by the pass that builds it
-  DevBuf distinct;              // plan_samples_per_cell: hash table of (CF plane, cell) and two counts
   double per_cell = 0;          // samples per CF plane and footprint, 0: not asked for
   int pos_mode = 0;             // its order: 1 position then CF index; 2 CF plane, position, offset
   int pl_fs = 0;                // plane-major records: grid_pl_block of their CF table
